@@ -1065,7 +1065,9 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	bb.st_offset = ctx->d_stoffset.as<int32_t>();
 	if (P.mbdof && P.nmps > 0) {
 		// each micropolygon's staging bound, computed once instead of in every tile it may reach
-		AQH_TRY(ctx->d_mpb.ensure(sizeof(int4) * (size_t)P.nmps), "alloc staging bounds");
+		// (followed by its path where some grid has two keys and none has more)
+		bb.mp_stride = fp.max_keys == 2 ? 2 : 1;
+		AQH_TRY(ctx->d_mpb.ensure(sizeof(int4) * (size_t)P.nmps * bb.mp_stride), "alloc staging bounds");
 		bb.mp_bounds = ctx->d_mpb.as<int4>();
 	}
 	const size_t nstore = store_size((long long)fp.sw * fp.sh, fp.spp);
@@ -1304,7 +1306,7 @@ static aqh_status enqueue_frame(aqh_ctx* ctx, RenderPlan& P, bool batched, bool 
 		launch_st_count(fp, P.g, P.bb, s);
 		launch_scan_i32(P.bb.st_count, P.bb.st_offset, P.nst * P.bb.nranges, nullptr, s);
 		launch_st_write(fp, P.g, P.bb, s);
-		if (P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, s);
+		if (P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, P.bb.mp_stride, s);
 	} else {
 		AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
 	}
@@ -1380,7 +1382,7 @@ static aqh_status render_plain(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 	P.bb.st_list = ctx->d_stlist.as<int32_t>();
 	P.bb.list_capacity = ctx->d_stlist.cap / sizeof(int32_t);
 	if (P.g.ngrids > 0) launch_st_write(fp, P.g, P.bb, s);
-	if (P.g.ngrids > 0 && P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, s);
+	if (P.g.ngrids > 0 && P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, P.bb.mp_stride, s);
 	if (P.g.ngrids <= 0) AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
 	for (int attempt = 0; attempt < 4; ++attempt) {
 		if (P.pool.capacity > 0) {

@@ -183,6 +183,7 @@ struct BinBuffers {
 	                       // micropolygon column, [32, 63) of each row (lo | hi << 16, int16 each);
 	                       // word 63 = 1 when present (one motion key, cu and cv at most 31)
 	int4* mp_bounds;       // motion frames, per micropolygon: its staging bound (pack_stage_bound), or null
+	int mp_stride;         // int4 entries per micropolygon: 1, or 2 with its path (pack_stage_path) second
 	int nranges;
 	int range_size;
 	int64_t list_capacity;
@@ -231,7 +232,8 @@ void launch_st_write(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cu
 // waits for (on an opaque frame, the resolve after the sampler), with
 // cudaStreamWaitEvent flags `wait_flags` (cudaEventWaitExternal in a capture).
 // Staging bound of every micropolygon of a motion blur / depth of field frame.
-void launch_mb_stage_bounds(const FrameParams& fp, const GridsDev& g, int4* out, cudaStream_t s);
+// `stride` 2: each bound is followed by the micropolygon's path (frames of at most two keys).
+void launch_mb_stage_bounds(const FrameParams& fp, const GridsDev& g, int4* out, int stride, cudaStream_t s);
 void launch_sample_tiles(const FrameParams& fp, const GridsDev& g, const SamplerDev& sm, const BinBuffers& b,
                          SampleStore st, FragPool pool, int32_t* err, cudaStream_t s,
                          cudaEvent_t colours_ready = nullptr, unsigned wait_flags = 0);

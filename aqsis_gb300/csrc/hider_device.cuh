@@ -304,16 +304,91 @@ struct MbStageBound {
 	float mnz, mxz;
 	bool keep;
 };
-__device__ __forceinline__ MbStageBound mb_stage_bound(const FrameParams& fp, const GridsDev& g, int gid, int m) {
+// With `path` (grids of one or two keys), also the same rectangle at each key
+// (pack_stage_path): the micropolygon's points move on straight lines between
+// the two, so at a fraction f of the way every sample that can hit it lies in
+// the rectangle interpolated at f.  A path is unbounded (both rectangles
+// everything) where that does not hold or cannot be packed: coordinates out
+// of the int16 range, and, under depth of field, a depth range that reaches z
+// = 0, where the circle of confusion is not largest at the range's ends.
+__device__ __forceinline__ int4 pack_stage_path(const float mn[2][2], const float mx[2][2], float gx, float gy,
+                                                bool ok) {
+	auto c = [&](float v, bool up) -> int {
+		ok = ok && v >= -32000.0f && v <= 32000.0f;  // false for NaN as well
+		return ok ? (up ? lceil_f(v) + 1 : (int)floorf(v) - 1) : 0;
+	};
+	int q[8];
+#pragma unroll
+	for (int k = 0; k < 2; ++k) {
+		q[4 * k] = c(mn[k][0] - gx, false);
+		q[4 * k + 1] = c(mx[k][0] + gx, true);
+		q[4 * k + 2] = c(mn[k][1] - gy, false);
+		q[4 * k + 3] = c(mx[k][1] + gy, true);
+	}
+	auto w = [&](int lo, int hi) -> int {
+		return ok ? (lo & 0xffff) | (hi << 16) : (int)0x7fff8000u;  // [-32768, 32767]
+	};
+	return make_int4(w(q[0], q[1]), w(q[2], q[3]), w(q[4], q[5]), w(q[6], q[7]));
+}
+
+// Narrows the range [fa, fb] of path fractions f to where lo(f) = lo0 + f
+// (lo1 - lo0) < x1 and hi(f) > x0, give or take 1/512 (the quotients are
+// approximate); an empty range has fa > fb.
+__device__ __forceinline__ void path_clip(float lo0, float lo1, float hi0, float hi1, float x0, float x1, float& fa,
+                                          float& fb) {
+	constexpr float kSlack = 1.0f / 512.0f;
+	auto half = [&](float a, float d) {  // a + f d <= 0
+		if (a > 0.0f || a + d > 0.0f) {
+			if (a > 0.0f && a + d > 0.0f) {
+				fa = 2.0f;
+				fb = -1.0f;
+			} else {
+				const float q = __fdividef(-a, d);
+				if (d > 0.0f) fb = fminf(fb, q + kSlack);
+				else fa = fmaxf(fa, q - kSlack);
+			}
+		}
+	};
+	half(lo0 - x1, lo1 - lo0);
+	half(x0 - hi0, hi0 - hi1);
+}
+
+// Does the path meet the tile at some fraction of the way?
+__device__ __forceinline__ bool path_meets(int4 p, int tpx0, int tpx1, int tpy0, int tpy1) {
+	auto lo = [](int w) -> float { return (float)(int)(int16_t)(w & 0xffff); };
+	auto hi = [](int w) -> float { return (float)(w >> 16); };
+	float fa = 0.0f, fb = 1.0f;
+	path_clip(lo(p.x), lo(p.z), hi(p.x), hi(p.z), (float)tpx0, (float)tpx1, fa, fb);
+	path_clip(lo(p.y), lo(p.w), hi(p.y), hi(p.w), (float)tpy0, (float)tpy1, fa, fb);
+	return fa <= fb;
+}
+
+__device__ __forceinline__ MbStageBound mb_stage_bound(const FrameParams& fp, const GridsDev& g, int gid, int m,
+                                                       int4* path = nullptr) {
 	const int cu = __ldg(g.cu + gid), nk = __ldg(g.nkeys + gid);
 	const long long nv = (long long)(cu + 1) * (__ldg(g.cv + gid) + 1);
 	const long long pb = __ldg(g.pbase + gid);
 	const int iv = m / cu, iu = m - iv * cu;
 	const int index = iv * (cu + 1) + iu;
 	float mnx = FLT_MAX, mny = FLT_MAX, mnz = FLT_MAX, mxx = -FLT_MAX, mxy = -FLT_MAX, mxz = -FLT_MAX;
+	float pmn[2][2], pmx[2][2];
+	bool finite = true;
 	for (int k = 0; k < nk; ++k) {
 		const long long kb = pb + k * nv + index;
 		const V3f a = ld3(g.P, kb), b = ld3(g.P, kb + 1), c = ld3(g.P, kb + cu + 1), d = ld3(g.P, kb + cu + 2);
+		if (path) {
+			// NaN coordinates drop out of the minima: checked on their sum
+			const float sum = ((a.x + b.x) + (c.x + d.x)) + ((a.y + b.y) + (c.y + d.y)) + ((a.z + b.z) + (c.z + d.z));
+			finite = finite && sum == sum;
+#pragma unroll
+			for (int e = 0; e < 2; ++e)
+				if (k == e || nk == 1) {
+					pmn[e][0] = fminf(fminf(a.x, b.x), fminf(c.x, d.x));
+					pmn[e][1] = fminf(fminf(a.y, b.y), fminf(c.y, d.y));
+					pmx[e][0] = fmaxf(fmaxf(a.x, b.x), fmaxf(c.x, d.x));
+					pmx[e][1] = fmaxf(fmaxf(a.y, b.y), fmaxf(c.y, d.y));
+				}
+		}
 		mnx = amin(mnx, amin(amin(amin(a.x, b.x), c.x), d.x));
 		mny = amin(mny, amin(amin(amin(a.y, b.y), c.y), d.y));
 		mnz = amin(mnz, amin(amin(amin(a.z, b.z), c.z), d.z));
@@ -331,6 +406,7 @@ __device__ __forceinline__ MbStageBound mb_stage_bound(const FrameParams& fp, co
 	}
 	const bool cropped = (mxx + gx) < fp.cull_x0 || (mxy + gy) < fp.cull_y0 || (mnx - gx) > fp.cull_x1 ||
 	                     (mny - gy) > fp.cull_y1;
+	if (path) *path = pack_stage_path(pmn, pmx, gx, gy, finite && nk <= 2 && (!fp.use_dof || (mnz > 0.0f && mxz < FLT_MAX)));
 	MbStageBound r;
 	r.x0 = (int)floorf(mnx - gx) - 1;
 	r.x1 = lceil_f(mxx + gx) + 1;

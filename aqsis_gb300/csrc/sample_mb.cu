@@ -628,12 +628,14 @@ __device__ __forceinline__ bool stage_mb(const FrameParams& fp, const GridsDev& 
 			}
 			(void)nk;
 			// conservative pixel rectangle over every time slice and lens stratum
-			const MbStageBound sb = bb.mp_bounds ? unpack_stage_bound(bb.mp_bounds[__ldg(g.mpbase + gid) + m])
-			                                     : mb_stage_bound(fp, g, gid, m);
+			const int4* pb = bb.mp_bounds ? bb.mp_bounds + (__ldg(g.mpbase + gid) + m) * bb.mp_stride : nullptr;
+			const MbStageBound sb = pb ? unpack_stage_bound(__ldg(pb)) : mb_stage_bound(fp, g, gid, m);
 			const float mnz = sb.mnz, mxz = sb.mxz;
 			const int sX = max(sb.x0, tpx0), eX = min(sb.x1, tpx1);
 			const int sY = max(sb.y0, tpy0), eY = min(sb.y1, tpy1);
 			active = sb.keep && sX < eX && sY < eY;
+			// its rectangle over the whole shutter meets the tile: does it at any time?
+			if (active && pb && bb.mp_stride == 2) active = path_meets(__ldg(pb + 1), tpx0, tpx1, tpy0, tpy1);
 			if (active && blk) {
 				float zmax = -FLT_MAX;
 				for (int y = sY; y < eY; ++y)
@@ -1048,6 +1050,42 @@ __device__ __forceinline__ bool mb_item(const FrameParams& fp, const Shutter& sh
 	return it.sX < it.eX && it.sY < it.eY && it.j0 < it.j1;
 }
 
+// The slices of a two-key micropolygon that can hold a hit in the tile: `div`
+// slices in, the first one and their number out.  Its points move on straight
+// lines between the keys (and rest before the first and after the last), so
+// it meets the tile only at path fractions [fa, fb] (path_clip on the key
+// bounds, grown by the largest circle of confusion and one pixel), and a
+// sample is tested in the slices whose window holds its time.  Slice b's
+// window is [open + b dt, open + (b + 1) dt] up to the rounding of the
+// accumulated times, which is below 0.04 dt for at most 256 slices of a
+// shutter no further than eight of its lengths from time 0; other shutters
+// and depth ranges that reach z = 0 under depth of field keep every slice.
+// With the path test at staging: 1080p motion blur + depth of field 202.6 ->
+// 182.0 ms, 640x480 motion blur 6.91 -> 6.45 ms (a tile is 7 to 11 pixels
+// wide, a path up to 20 long: before, each tile its box met staged the
+// micropolygon and all of its slices).
+template <class R>
+__device__ __forceinline__ void tile_slices(const FrameParams& fp, const Shutter& sh, const R& r, int tpx0, int tpy0,
+                                            int tpx1, int tpy1, int& b0, int& div) {
+	const float len = sh.close - sh.open, span = r.kt[1] - r.kt[0];
+	if (!(len > 0.0f) || !(fmaxf(fabsf(sh.open), fabsf(sh.close)) <= 8.0f * len) || !(span > 0.0f)) return;
+	if (fp.use_dof && !(r.bmn[2] > 0.0f && r.bmx[2] < FLT_MAX)) return;
+	float fa = 0.0f, fb = 1.0f;
+	const float mx = r.cocmax[0] + 1.0f, my = r.cocmax[1] + 1.0f;
+	path_clip(r.kbmn[0][0] - mx, r.kbmn[1][0] - mx, r.kbmx[0][0] + mx, r.kbmx[1][0] + mx, (float)tpx0, (float)tpx1, fa, fb);
+	path_clip(r.kbmn[0][1] - my, r.kbmn[1][1] - my, r.kbmx[0][1] + my, r.kbmx[1][1] + my, (float)tpy0, (float)tpy1, fa, fb);
+	if (fa > fb) {
+		div = 0;
+		return;
+	}
+	const float inv_dt = (float)div / len;
+	int last = div - 1;
+	if (fa > 0.0f) b0 = max(0, (int)fminf((r.kt[0] + fa * span - sh.open) * inv_dt - 1.05f, 256.0f));
+	if (fb < 1.0f) last = (int)fmaxf(fminf((r.kt[0] + fb * span - sh.open) * inv_dt + 0.05f, (float)last), -1.0f);
+	div = max(0, last + 1 - b0);
+	b0 = min(b0, 255);
+}
+
 // Lens offset of the sample of lens stratum k in lens pattern dp
 // (projectToCircle of the pattern's [0,1)^2 lens sample, imagepixel.cpp:338-347).
 __device__ __forceinline__ float2 lens_offset(const SamplerDev& smp, int dp, int spp, int k) {
@@ -1102,6 +1140,7 @@ struct SmemQT {
 	MbRecT<NK> rec[SLOTS];
 	int2 pend[SLOTS];
 	int pref[SLOTS + 1];                  // running count of (candidate, slice) items
+	uint8_t slice0[SLOTS];                // first slice of each candidate's items
 	ItemQ items[kItemsQ];
 	int ipref[kItemsQ + 1];               // running count of the kept items' sample slots
 	int qgrid[kThreadsQ];
@@ -1306,7 +1345,13 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 			const int2 e = sm.pend[t];
 			MbRec& rr = sm.rec[t];
 			build_mb_record(fp, g, e.x, e.y, rr);
-			nitems = (rr.nkeys > 1) ? motion_divisions(rr, sh.timeRanges) : 1;
+			int b0 = 0;
+			nitems = 1;
+			if (rr.nkeys > 1) {
+				nitems = motion_divisions(rr, sh.timeRanges);
+				if (rr.nkeys == 2 && !any_nan) tile_slices(fp, sh, rr, tpx0, tpy0, tpx1, tpy1, b0, nitems);
+			}
+			sm.slice0[t] = (uint8_t)b0;
 		}
 		int total;
 		const int pre = block_excl_sum(sm.warp_tot, nitems, total);
@@ -1325,7 +1370,7 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 				}
 				const MbRec& r = sm.rec[lo];
 				MbItem it;
-				if (!mb_item(fp, sh, r, slice_times, p - sm.pref[lo], sm.dext, tpx0, tpy0, tpx1, tpy1, it)) continue;
+				if (!mb_item(fp, sh, r, slice_times, sm.slice0[lo] + p - sm.pref[lo], sm.dext, tpx0, tpy0, tpx1, tpy1, it)) continue;
 				// early-z of the whole item: behind every sample of its pixels at the
 				// round's start, so that every one of its slots would fail the
 				// per-sample test below

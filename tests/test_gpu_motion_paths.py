@@ -1,0 +1,58 @@
+"""The motion sampler's pruning of tiles and time slices by a micropolygon's
+path, and its replay of flagged samples, against the oracle (exact: both only
+leave out tests that cannot hit).  Frames are several tiles wide, so paths
+start, end, cross and graze tiles; each case moves its grids differently."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from aqsis_gb300 import scene as S
+from tests.test_gpu_parity import compare
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(shutter=(0.0, 1.0), times=(0.0, 1.0), move=(30.0, 4.0), dof=False, z=(1.0, 50.0), shear=0.0, static=0.3,
+           xs=4, ys=4, flat=False, crop=None, seed=0):
+    """Two-key grids over a 72x56 frame, each displaced along `move` turned by a
+    random angle, key 1 sheared by `shear`; a share `static` has one key."""
+    rng = np.random.default_rng(seed)
+    fr = S.Frame(width=72, height=56, xsamples=xs, ysamples=ys, q_dither=0.0, shutter=shutter, crop=crop)
+    if dof:
+        fr.fstop, fr.focal_length, fr.focal_distance, fr.dof_scale = 2.8, 0.4, 20.0, (40.0, 40.0)
+    parts = []
+    for i in range(40):
+        n = int(rng.integers(1, 9))
+        g = S.regular_grids(1, 72, 56, rng, n=n, zrange=z, slope=0.0 if flat else 0.02, motion=1.0,
+                            origin_margin=10.0)
+        P = g.P.reshape(2, -1, 4)
+        a = rng.uniform(0, 2 * np.pi)
+        d = np.array([np.cos(a) * move[0] - np.sin(a) * move[1], np.sin(a) * move[0] + np.cos(a) * move[1]])
+        P[1, :, :2] = P[0, :, :2] + d + shear * (P[0, :, :2] - P[0, 0, :2])[:, ::-1]
+        if flat:
+            P[:, :, 2] = float(rng.integers(2, 5))   # coplanar layers: depths tie and round below their bounds
+        if rng.random() < static:
+            g = dataclasses.replace(g, P=P[0].copy(), nkeys=np.ones(1, np.int32), times=np.zeros(1, np.float32),
+                                    tbase=np.zeros(1, np.int32))
+        else:
+            g = dataclasses.replace(g, P=P.reshape(-1, 4), times=np.array(times, np.float32))
+        parts.append(g)
+    return S.Scene(fr, S.concat_grids(parts), S.make_samples(fr, rng, 50))
+
+
+CASES = {
+    "long": dict(), "short": dict(move=(0.3, 0.0)), "rest": dict(move=(0.0, 0.0)), "huge": dict(move=(4000.0, 0.0)),
+    "beyond_int16": dict(move=(90000.0, 3.0)), "shear": dict(shear=0.8, move=(9.0, 2.0)),
+    "keys_inside_shutter": dict(times=(0.3, 0.6)), "keys_around_shutter": dict(times=(-1.0, 3.0)),
+    "late_shutter": dict(shutter=(100.0, 100.5), times=(100.0, 100.5)), "reversed_keys": dict(times=(1.0, 0.0)),
+    "dof": dict(dof=True, move=(12.0, 1.0)), "dof_depth_reaches_zero": dict(dof=True, z=(-0.05, 0.05), move=(8.0, 0.0)),
+    "samples_1x1": dict(xs=1, ys=1), "samples_16x16": dict(xs=16, ys=16, move=(10.0, 0.0)), "samples_5x3": dict(xs=5, ys=3),
+    "crop": dict(crop=(13, 61, 9, 40)), "flat": dict(flat=True), "flat_dof": dict(flat=True, dof=True, move=(6.0, 0.0)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_moving_frame_matches_oracle(hider, oracle, name):
+    sc = _scene(seed=sorted(CASES).index(name), **CASES[name])
+    compare(hider.render_scene(sc), oracle.render(sc), exact_pixels=True)
