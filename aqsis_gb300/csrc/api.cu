@@ -1018,12 +1018,10 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	fp.max_keys = max_keys;
 	fp.any_motion = motion ? 1 : 0;
 	P.mbdof = fp.use_dof || fp.any_motion;
-	// opaque motion blur / depth of field frames sample smaller tiles (two
-	// CTAs share an SM); frames that keep fragments use the default size
-	const bool frags = ctx->any_transparent || !fp.cullable || fp.midpoint_store || ctx->csg_n > 0;
+	// the parallel motion sampler takes smaller tiles (two CTAs share an SM)
 	int tile_pixels = ctx->tune.tile_pixels;
-	if (P.mbdof && !frags) {
-		const int cap = sample_mb_opaque_tile_pixels(fp.spp);
+	if (P.mbdof && sample_mb_parallel(fp, ctx->csg_n > 0)) {
+		const int cap = sample_mb_parallel_tile_pixels(fp.spp);
 		tile_pixels = tile_pixels > 0 ? std::min(tile_pixels, cap) : cap;
 	}
 	set_tiling(fp, tile_pixels, ctx->tune.supertile_pixels);

@@ -168,7 +168,7 @@ struct FragPool {
 	int32_t* overflow;
 	int32_t* occluders;  // nonzero when some micropolygon may be occluding (opaque or matte alpha)
 	int32_t* heads;      // fragment-only frames: each sample's list head, pixel-major ([pixel][sample
-	                     // index]), handed to resolve_frag_kernel; null: the sampler resolves in place
+	                     // index]), handed to the Combine kernels of sample.cu; null: the sampler resolves in place
 };
 
 struct BinBuffers {
@@ -256,8 +256,9 @@ void launch_sample_mb(const FrameParams& fp, const GridsDev& g, const SamplerDev
                       SampleStore st, FragPool pool, const float4* dof_bounds, const float* slice_times,
                       cudaStream_t s);
 void slice_times_h(float open, float close, int spp, std::vector<float>& out);
-// Largest sampling tile (pixels) of opaque motion blur / depth of field frames.
-int sample_mb_opaque_tile_pixels(int spp);
+// Motion blur / depth of field frames the parallel sampler takes, and its largest tile (pixels).
+bool sample_mb_parallel(const FrameParams& fp, bool csg);
+int sample_mb_parallel_tile_pixels(int spp);
 void static_tiling(FrameParams& fp, int tile_pixels);
 // Frame options resolved from an aqh_frame_desc (plus the host filter table).
 aqh_status resolve_frame(const aqh_frame_desc& d, FrameParams& fp, std::vector<float>& ftab, std::string& err);

@@ -321,6 +321,28 @@ __device__ __forceinline__ void key_data(const GridsDev& g, const FragPool& pool
 	}
 }
 
+// A list holding a NaN depth has no sorted order: the selection above then
+// depends on the order of the walk.  Relinks such a list newest (largest id)
+// first, the insertion order, whichever order the sampler appended in;
+// entries with equal ids carry the same data.  Returns the new head.
+static __device__ __noinline__ int list_newest_first(const float4* frag, int32_t* next, int head) {
+	int out = -1;
+	for (int f = head; f >= 0;) {
+		const int nx = next[f];
+		const int id = __float_as_int(frag[f].y);
+		int before = -1, at = out;
+		while (at >= 0 && __float_as_int(frag[at].y) > id) {
+			before = at;
+			at = next[at];
+		}
+		next[f] = at;
+		if (before < 0) out = f;
+		else next[before] = f;
+		f = nx;
+	}
+	return out;
+}
+
 constexpr int kCombineLocal = 24;  // lists up to this long are sorted in local memory
 
 // CqImagePixel::Combine for a sample with transparent fragments
@@ -379,6 +401,7 @@ __device__ __forceinline__ int combine_fragments_t(const FrameParams& fp, const 
 	// short lists are now sorted; long ones (or NaN depths) are walked in
 	// order by selection
 	const bool local = ntot <= kCombineLocal && !nan;
+	if (nan) head = list_newest_first(pool.frag, pool.next, head);
 	if (CSG && any_csg && !local && g.csg.overflow) atomicOr(g.csg.overflow, 1);  // CSG needs the sorted list held
 	if (local) {
 		if (has_occl) insert(occl[6], 0x7fffffff, 1, -1);

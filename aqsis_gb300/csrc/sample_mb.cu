@@ -11,11 +11,12 @@
 // time slice whose window holds the sample's time (and, without depth of
 // field, whose sample-index range holds the sample); with depth of field each
 // sample belongs to one lens stratum, whose shifted bound decides whether the
-// reference visits it.  Frames with transparency (sample_mb_kernel) walk each
-// sample's candidates in insertion order, one sample per lane, finding the
-// slices by binary search in a per-frame table of the reference's accumulated
-// slice times; opaque frames (sample_mbq_kernel) test (slice, sample) pairs in
-// parallel and fold the hits (see the section on opaque frames).
+// reference visits it.  sample_mbq_kernel tests (slice, sample) pairs in
+// parallel and folds the hits (see its section); frames that section does not
+// cover (CSG solids, a z display with the max, average or midpoint depth
+// filter) take sample_mb_kernel, which walks each sample's candidates in
+// insertion order, one sample per lane, finding the slices by binary search in
+// a per-frame table of the reference's accumulated slice times.
 #include "aqh_internal.h"
 #include "hider_device.cuh"
 #include "sample_common.cuh"
@@ -907,7 +908,7 @@ sample_mb_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Samp
 }
 
 
-// ---- opaque frames: parallel (slice, sample) tests with an ordered replay ----
+// ---- parallel (slice, sample) tests with an ordered replay ----
 //
 // The order argument of the static opaque kernel (sample.cu) carries over:
 // RenderMPG_MBOrDof skips a (slice, sample) test when the slice's bound has
@@ -924,6 +925,18 @@ sample_mb_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Samp
 // queue it for the full hit test, 32 at a time, whose hits fold into a
 // 64-bit shared-memory atomicMin.  Hits below their slice's min.z, NaN or
 // zero depths flag the sample for an in-order replay from the round's start.
+//
+// TRANSP frames (some micropolygon not opaque) take each round's items in two
+// passes, the occluding candidates' and then the transparent ones'.  The
+// reference keeps a transparent hit when !(b > z) and !(z <= D), b its slice's
+// min z and z the occlZ at its place in insertion order.  Only occluding hits
+// move z, so it lies between the round's start (prev) and, of a sample no
+// occluding hit flagged, the round's end (key): where the two decide alike the
+// hit is a fragment or not, and where they differ the warp takes z from the
+// sample's occluding hits of the candidates before it.  Flagged samples
+// replay both kinds in order.  640x480, 16 samples, motion blur + depth of
+// field, half of one layer transparent: 16.6 ms on the ordered kernel (one
+// sample per lane, slices one after another, one CTA per SM), 4.7 ms here.
 __device__ __forceinline__ unsigned long long depth_key_m(float z, int w) {
 	const uint32_t u = __float_as_uint(z);
 	const uint32_t o = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -1106,6 +1119,7 @@ constexpr int kItemsQ = 192;     // kept (candidate, slice) items per pass (at m
 constexpr int kTileSampQ = 2048;
 constexpr int kTilePixQ = 256;
 constexpr int kBinsQ = 64;       // time bins of a pixel at most
+constexpr int kFragRunQ = 64;    // pool slots a warp reserves at a time (at least 32: one drain's hits)
 constexpr int kBinTabQ = kTileSampQ + kTilePixQ;  // (bins + 1) entries per pixel, over the tile
 
 // One kept (candidate, slice) item of a pass.  Its sample slots are the
@@ -1124,7 +1138,7 @@ struct ItemQ {
 	uint32_t mnpix, mrw;  // ceil(2^32 / npix), ceil(2^32 / rw) (0 for 1): exact quotients of slot indices
 };
 
-template <int NK, int SLOTS>
+template <int NK, int SLOTS, bool TRANSP>
 struct SmemQT {
 	unsigned long long key[kTileSampQ];   // occluding hit of each tile sample (depth_key_m)
 	unsigned long long prev[kTileSampQ];  // ... at the start of the round
@@ -1154,15 +1168,21 @@ struct SmemQT {
 	int warp_tot[32];
 	int first_reject, qn, nsurv, any_nan;
 	float dext[4];                        // min dofb[.][0], min [.][1], max [.][2], max [.][3]
+	int32_t fhead[TRANSP ? kTileSampQ : 1];  // fragment list of each tile sample
 };
 
-// candidates per round: 64 four-key records, or 96 two-key ones in less space
-constexpr int kSlotsQ2 = 96;
-using SmemQ = SmemQT<kMaxKeys, kSlotsQ>;
-using SmemQ2 = SmemQT<2, kSlotsQ2>;
+// candidates per round: 64 four-key records, or 96 two-key ones in less space;
+// with fragment lists 32 and 64
+constexpr int kSlotsQ2 = 96, kSlotsQT = 32, kSlotsQ2T = 64;
+using SmemQ = SmemQT<kMaxKeys, kSlotsQ, false>;
+using SmemQ2 = SmemQT<2, kSlotsQ2, false>;
+using SmemQT4 = SmemQT<kMaxKeys, kSlotsQT, true>;
+using SmemQT2 = SmemQT<2, kSlotsQ2T, true>;
 // two CTAs per SM: 228 KB of shared memory less 1 KB reserved per CTA
 static_assert(sizeof(SmemQ) <= (228 * 1024 - 2 * 1024) / 2, "two opaque motion CTAs must fit on an SM");
 static_assert(sizeof(SmemQ2) <= sizeof(SmemQ), "two-key rounds must fit where four-key ones do");
+static_assert(sizeof(SmemQT4) <= (228 * 1024 - 2 * 1024) / 2 && sizeof(SmemQT2) <= (228 * 1024 - 2 * 1024) / 2,
+              "two transparent motion CTAs must fit on an SM");
 static_assert(kSlotsQ2 <= kThreadsQ && kSlotsQ2 < 256, "one record per thread; slots fit 8 bits");
 
 // One (slice, sample) test as RenderMPG_MBOrDof makes it, given occlZ:
@@ -1171,15 +1191,71 @@ template <class R>
 __device__ __forceinline__ bool mb_slice_test(const FrameParams& fp, const R& r, const Bnd& B, bool moving,
                                               float time0, float time1, const float* dofb_k, int px, int py,
                                               float x, float y, float stime, float sdx, float sdy, float oz,
-                                              float& D, const float4* tri, const GridsDev* gt) {
+                                              float& D, float& u, float& v, const float4* tri, const GridsDev* gt) {
 	if (moving && (stime < time0 || stime > time1)) return false;
 	const Bnd TB = fp.use_dof ? stratum_bound(fp, B, dofb_k) : B;
 	if (px < (int)floorf(TB.mnx) || px >= lceil_f(TB.mxx) || py < (int)floorf(TB.mny) || py >= lceil_f(TB.mxy))
 		return false;
 	if ((x < TB.mnx || x > TB.mxx) || (y < TB.mny || y > TB.mxy)) return false;
 	if (B.mnz > oz) return false;
-	float u, v;
 	return mb_sample(fp, r, moving, fp.use_dof != 0, x, y, stime, sdx, sdy, D, u, v, tri, gt);
+}
+
+// Every test RenderMPG_MBOrDof makes of sample j of pixel (px, py) against
+// candidate r with occlZ at `oz`: the number of slices that hit it past
+// early-z, with the depth and (u, v) of the hit (the same in every slice) and
+// the least min z of those slices (a NaN min z never fails early-z: -inf).
+// For the ordered passes, which call it for few samples: kernels with fragments
+// do so from three places and call it out of line (mb_hits_call), which keeps
+// their hot loops' registers.
+template <class R>
+__device__ __forceinline__ int mb_hits(const FrameParams& fp, const GridsDev& g, const SamplerDev& smp,
+                                    const BinBuffers& bb, const R& r, const float* slice_times, const float* dk,
+                                    int px, int py, int j, float2 pos, float stime, float2 lens, float oz, float& D,
+                                    float2& uv, float& bz) {
+	const Shutter sh = shutter_of(fp);
+	const bool moving = r.nkeys > 1;
+	const int div = moving ? motion_divisions(r, sh.timeRanges) : 1;
+	const float dt = (sh.close - sh.open) / div;
+	const float* T = slice_times + (div * (div - 1)) / 2;
+	int b0 = 0, b1 = 0, n = 0;
+	if (moving) {
+		// slices whose window can hold the sample's time, in slice order
+		int blo = 0, bhi = div - 1;
+		while (blo < bhi) {
+			const int mid = (blo + bhi + 1) >> 1;
+			if (T[mid] - dt <= stime) blo = mid; else bhi = mid - 1;
+		}
+		b1 = blo;
+		b0 = b1;
+		while (b0 > 0 && (T[b0] - dt) >= stime) --b0;
+		if (stime != stime) { b0 = 0; b1 = div - 1; }  // a NaN time passes every window test
+	}
+	for (int sb = b0; sb <= b1; ++sb) {
+		Bnd B;
+		float time0, time1, Ds, u, v;
+		int j0, j1;
+		if (!mb_slice(fp, sh, r, T, div, dt, sb, B, time0, time1, j0, j1)) continue;
+		if (j < j0 || j >= j1) continue;
+		if ((r.bits & 8) && lod_rejects(fp, g, smp, r.grid, px, py, j)) continue;
+		if (!mb_slice_test(fp, r, B, moving, time0, time1, dk, px, py, pos.x, pos.y, stime, lens.x, lens.y, oz, Ds, u,
+		                   v, bb.tri, &g))
+			continue;
+		const float b = (B.mnz != B.mnz) ? -INFINITY : B.mnz;
+		bz = n > 0 ? fminf(bz, b) : b;
+		D = Ds;
+		uv = make_float2(u, v);
+		++n;
+	}
+	return n;
+}
+
+template <class R>
+__device__ __noinline__ int mb_hits_call(const FrameParams& fp, const GridsDev& g, const SamplerDev& smp,
+                                         const BinBuffers& bb, const R& r, const float* slice_times, const float* dk,
+                                         int px, int py, int j, float2 pos, float stime, float2 lens, float oz, float& D,
+                                         float2& uv, float& bz) {
+	return mb_hits(fp, g, smp, bb, r, slice_times, dk, px, py, j, pos, stime, lens, oz, D, uv, bz);
 }
 
 __device__ __forceinline__ uint32_t quot_magic(int d) {
@@ -1189,11 +1265,12 @@ __device__ __forceinline__ uint32_t quot_magic(int d) {
 // is exact there (the rounding up adds less than r * d / 2^32 / d < 1 / d)
 __device__ __forceinline__ int quot(int r, uint32_t m) { return m == 0u ? r : (int)__umulhi((unsigned)r, m); }
 
-template <int NK, int SLOTS>
+template <int NK, int SLOTS, bool TRANSP>
 __global__ void __launch_bounds__(kThreadsQ, 2)
-sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, SampleStore st,
-                  const float4* dof_bounds, const float* slice_times) {
-	using SmemQ = SmemQT<NK, SLOTS>;
+sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant__ GridsDev g,
+                  const __grid_constant__ SamplerDev smp, const __grid_constant__ BinBuffers bb, SampleStore st,
+                  FragPool pool, const float4* dof_bounds, const float* slice_times) {
+	using SmemQ = SmemQT<NK, SLOTS, TRANSP>;
 	using MbRec = MbRecT<NK>;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	SmemQ& sm = *reinterpret_cast<SmemQ*>(smem_raw);
@@ -1228,6 +1305,7 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 		sm.key[i] = kinit;
 		sm.prev[i] = kinit;
 		sm.kinv[i] = (uint8_t)(i % spp);
+		if (TRANSP) sm.fhead[i] = -1;
 	}
 	for (int i = t; i < kTileSampQ / 32; i += kThreadsQ) {
 		sm.flag[i] = 0u;
@@ -1330,6 +1408,39 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 	__syncthreads();
 	const bool any_nan = sm.any_nan != 0;
 
+	// TRANSP: append fragments of the lanes with `app` (one per lane) to their
+	// samples' lists.  Pool slots come in runs of kFragRunQ a warp reserves with
+	// one atomic (a run's rest is used before the next is reserved).
+	unsigned long long rnext = 0;
+	int rleft = 0;
+	auto append = [&](bool app, int s, float D, int id, float u, float v) {
+		const unsigned bal = __ballot_sync(0xffffffffu, app);
+		const int nh = __popc(bal);
+		if (nh == 0) return;
+		unsigned long long base = 0;
+		if (nh > rleft) {
+			if (lane == 0) base = atomicAdd(pool.count, (unsigned long long)kFragRunQ);
+			base = __shfl_sync(0xffffffffu, base, 0);
+		}
+		if (app) {
+			const int rank = __popc(bal & ((1u << lane) - 1u));
+			const long long idx = (long long)(rank < rleft ? rnext + rank : base + (rank - rleft));
+			if (idx < pool.capacity) {
+				pool.frag[idx] = make_float4(D, __int_as_float(id), u, v);
+				pool.next[idx] = atomicExch(&sm.fhead[s], (int)idx);
+			} else {
+				atomicOr(pool.overflow, 1);
+			}
+		}
+		if (nh > rleft) {
+			rnext = base + (nh - rleft);
+			rleft = kFragRunQ - (nh - rleft);
+		} else {
+			rnext += nh;
+			rleft -= nh;
+		}
+	};
+
 	const int lbeg = bb.st_offset[st_idx * bb.nranges];
 	const int lend = (int)min((long long)bb.st_offset[(st_idx + 1) * bb.nranges], (long long)bb.list_capacity);
 	int lp = lbeg, r0 = 0, qtotal = 0, npend = 0;
@@ -1353,8 +1464,11 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 			}
 			sm.slice0[t] = (uint8_t)b0;
 		}
+		// TRANSP: the occluding candidates' items first, then the transparent ones'
+		const bool mine = t < npend && (!TRANSP || (sm.rec[t].bits & 2));
+		for (int ph = 0; ph < (TRANSP ? 2 : 1); ++ph) {
 		int total;
-		const int pre = block_excl_sum(sm.warp_tot, nitems, total);
+		const int pre = block_excl_sum(sm.warp_tot, (t < npend && mine == (ph == 0)) ? nitems : 0, total);
 		if (t < npend) sm.pref[t] = pre;
 		__syncthreads();
 
@@ -1434,23 +1548,63 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 			int qn = 0;
 			auto drain = [&](int n) {
 				// hit tests of queue entries [0, n), one per lane
+				bool app = false, amb = false;  // TRANSP, second pass: a fragment, or one if z allows
+				int s = 0, c = 0;
+				float D = 0.0f, u = 0.0f, v = 0.0f;
 				if (lane < n) {
 					const uint32_t e = wq[lane];
-					const int c = (int)(e & 0xffu), s = (int)(e >> 8);
+					c = (int)(e & 0xffu);
+					s = (int)(e >> 8);
 					const MbRec& r = sm.rec[c];
 					const int pl = s / spp, j = s - pl * spp;
 					const int px = tpx0 + pl % fp.tile_w, py = tpy0 + pl / fp.tile_w;
 					const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
 					const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s]);
-					float D, u, v;
 					if (!((r.bits & 8) && lod_rejects(fp, g, smp, r.grid, px, py, j)) &&
 					    mb_sample(fp, r, r.nkeys > 1, usingDof, (float)px + o.x, (float)py + o.y, sm.stime[s], d.x, d.y,
 					              D, u, v, bb.tri, &g)) {
-						if (!(D >= wz[lane]) || D == 0.0f)
+						if (TRANSP && ph == 1) {
+							// kept when !(b > z) and !(z <= D) for the z of the ordered
+							// sequence, which lies between the round's start and its end
+							const float zp = key_depth_m(sm.prev[s]), zk = key_depth_m(sm.key[s]);
+							if (!(zp <= D)) {
+								app = !(wz[lane] > zk) && !(zk <= D);
+								amb = !app;
+							}
+						} else if (!(D >= wz[lane]) || D == 0.0f) {
 							atomicOr(&sm.flag[s >> 5], 1u << (s & 31));
-						else
+						} else {
 							atomicMin(&sm.key[s], depth_key_m(D, r.id));
+						}
 					}
+				}
+				if (TRANSP && ph == 1) {
+					// between the two: z from the occluding candidates before this one
+					uint32_t am = __ballot_sync(0xffffffffu, amb);
+					while (am) {
+						const int src = __ffs(am) - 1;
+						am &= am - 1u;
+						const int s_ = __shfl_sync(0xffffffffu, s, src), c_ = __shfl_sync(0xffffffffu, c, src);
+						const int pl = s_ / spp, j = s_ - pl * spp;
+						const int px = tpx0 + pl % fp.tile_w, py = tpy0 + pl / fp.tile_w;
+						const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
+						const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s_]);
+						float z = key_depth_m(sm.prev[s_]);
+						for (int c0 = 0; c0 < c_; c0 += 32) {
+							const int cc = c0 + lane;
+							float Dc, bz;
+							float2 uvc;
+							if (cc < c_ && (sm.rec[cc].bits & 2) &&
+							    mb_hits_call(fp, g, smp, bb, sm.rec[cc], slice_times, sm.dofb[sm.kinv[s_]], px, py, j,
+							            make_float2((float)px + o.x, (float)py + o.y), sm.stime[s_], d, INFINITY, Dc, uvc,
+							            bz) > 0)
+								z = fminf(z, Dc);
+						}
+#pragma unroll
+						for (int k = 16; k > 0; k >>= 1) z = fminf(z, __shfl_xor_sync(0xffffffffu, z, k));
+						if (lane == src) app = !(wz[lane] > z) && !(z <= D);
+					}
+					append(app, s, D, sm.rec[c].id, u, v);
 				}
 				__syncwarp();
 			};
@@ -1535,6 +1689,7 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 			drain(qn);
 			__syncthreads();
 		}
+		}  // occluding, transparent
 		int anyf = 0;
 		for (int i = t; i < nflagw; i += kThreadsQ) anyf |= (int)(sm.flag[i] != 0u);
 
@@ -1562,47 +1717,21 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 					const float stime = sm.stime[s];
 					const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s]);
 					const float* dk = sm.dofb[sm.kinv[s]];
+					const float2 xy = make_float2(x, y);
 					float oz = key_depth_m(sm.prev[s]);
 					int w = key_winner_m(sm.prev[s]);
 					for (int c0 = 0; c0 < npend; c0 += 32) {
 						const int c = c0 + lane;
-						bool hit = false;
 						float Dc = 0.0f, bz = 0.0f;
+						float2 uv = make_float2(0.0f, 0.0f);
+						bool hit = false;
 						if (c < npend) {
-							const MbRec& r = sm.rec[c];
-							const bool moving = r.nkeys > 1;
-							const int div = moving ? motion_divisions(r, sh.timeRanges) : 1;
-							const float dt = (sh.close - sh.open) / div;
-							const float* T = slice_times + (div * (div - 1)) / 2;
-							int b0 = 0, b1 = 0;
-							if (moving) {
-								// slices whose window can hold the sample's time, in slice order
-								int blo = 0, bhi = div - 1;
-								while (blo < bhi) {
-									const int mid = (blo + bhi + 1) >> 1;
-									if (T[mid] - dt <= stime) blo = mid; else bhi = mid - 1;
-								}
-								b1 = blo;
-								b0 = b1;
-								while (b0 > 0 && (T[b0] - dt) >= stime) --b0;
-								if (stime != stime) { b0 = 0; b1 = div - 1; }  // a NaN time passes every window test
-							}
-							for (int sb = b0; sb <= b1; ++sb) {
-								Bnd B;
-								float time0, time1;
-								int j0, j1;
-								if (!mb_slice(fp, sh, r, T, div, dt, sb, B, time0, time1, j0, j1)) continue;
-								if (j < j0 || j >= j1) continue;
-								if ((r.bits & 8) && lod_rejects(fp, g, smp, r.grid, px, py, j)) continue;
-								float D;
-								if (!mb_slice_test(fp, r, B, moving, time0, time1, dk, px, py, x, y, stime, d.x, d.y,
-								                   INFINITY, D, bb.tri, &g))
-									continue;
-								const float b = (B.mnz != B.mnz) ? -INFINITY : B.mnz;
-								bz = hit ? fminf(bz, b) : b;
-								Dc = D;
-								hit = true;
-							}
+							if (TRANSP)
+								hit = mb_hits_call(fp, g, smp, bb, sm.rec[c], slice_times, dk, px, py, j, xy, stime, d, INFINITY, Dc,
+								                   uv, bz) > 0;
+							else
+								hit = mb_hits(fp, g, smp, bb, sm.rec[c], slice_times, dk, px, py, j, xy, stime, d, INFINITY, Dc, uv,
+								              bz) > 0;
 						}
 						uint32_t hb = __ballot_sync(0xffffffffu, hit);
 						while (hb) {
@@ -1610,9 +1739,17 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 							hb &= hb - 1u;
 							const float Db = __shfl_sync(0xffffffffu, Dc, b);
 							const float bzb = __shfl_sync(0xffffffffu, bz, b);
-							if (!(bzb > oz) && !(oz <= Db)) {
+							if (bzb > oz || oz <= Db) continue;
+							if (!TRANSP || (sm.rec[c0 + b].bits & 2)) {
 								oz = Db;
 								w = sm.rec[c0 + b].id;
+							} else {
+								// a fragment for every slice that passes early-z
+								int nf = 0;
+								if (lane == b)
+									nf = mb_hits_call(fp, g, smp, bb, sm.rec[c], slice_times, dk, px, py, j, xy, stime, d, oz, Dc, uv, bz);
+								nf = __shfl_sync(0xffffffffu, nf, b);
+								for (int k = 0; k < nf; ++k) append(lane == b, s, Dc, sm.rec[c0 + b].id, uv.x, uv.y);
 							}
 						}
 					}
@@ -1661,15 +1798,19 @@ sample_mbq_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sam
 		const unsigned long long kk = sm.key[s];
 		const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
 		const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s]);
-		mb_resolve<false>(fp, g, FragPool{}, st, pix * spp + j, store_index(pix, j, spp), (float)px + o.x,
-		                  (float)py + o.y, sm.stime[s], d.x, d.y, key_depth_m(kk), key_winner_m(kk), -1);
+		mb_resolve<TRANSP>(fp, g, pool, st, pix * spp + j, store_index(pix, j, spp), (float)px + o.x, (float)py + o.y,
+		                   sm.stime[s], d.x, d.y, key_depth_m(kk), key_winner_m(kk), TRANSP ? sm.fhead[s] : -1);
 		if (st.wmask) st.wmask[store_index(pix, j, spp)] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
 	}
 }
 
 }  // namespace
 
-int sample_mb_opaque_tile_pixels(int spp) { return max(1, min(kTilePixQ, kTileSampQ / max(1, spp))); }
+// Frames whose samples are occlusion cullable by one occlZ, without solids:
+// the parallel sampler's order argument covers them.
+bool sample_mb_parallel(const FrameParams& fp, bool csg) { return fp.cullable && !fp.midpoint_store && !csg; }
+
+int sample_mb_parallel_tile_pixels(int spp) { return max(1, min(kTilePixQ, kTileSampQ / max(1, spp))); }
 
 size_t sample_mb_smem(bool transp) {
 	return sizeof(SmemM) + (transp ? sizeof(int32_t) * kTileSampM : 0);
@@ -1680,25 +1821,37 @@ void launch_sample_mb(const FrameParams& fp, const GridsDev& g, const SamplerDev
                       cudaStream_t s) {
 	const int ntiles = fp.ntx * fp.nty;
 	configure_sample_mb_kernels();
-	if (pool.capacity > 0)
+	// two-key records hold more candidates per round
+	const bool two = fp.max_keys >= 1 && fp.max_keys <= 2;
+	if (!sample_mb_parallel(fp, g.csg.nnodes > 0))
 		sample_mb_kernel<true><<<ntiles, kThreadsM, sample_mb_smem(true), s>>>(fp, g, sm, b, st, pool, dof_bounds,
 		                                                                      slice_times);
-	else if (fp.max_keys >= 1 && fp.max_keys <= 2)
-		sample_mbq_kernel<2, kSlotsQ2><<<ntiles, kThreadsQ, sizeof(SmemQ2), s>>>(fp, g, sm, b, st, dof_bounds,
-		                                                                       slice_times);
+	else if (pool.capacity > 0 && two)
+		sample_mbq_kernel<2, kSlotsQ2T, true><<<ntiles, kThreadsQ, sizeof(SmemQT2), s>>>(fp, g, sm, b, st, pool,
+		                                                                               dof_bounds, slice_times);
+	else if (pool.capacity > 0)
+		sample_mbq_kernel<kMaxKeys, kSlotsQT, true><<<ntiles, kThreadsQ, sizeof(SmemQT4), s>>>(
+		    fp, g, sm, b, st, pool, dof_bounds, slice_times);
+	else if (two)
+		sample_mbq_kernel<2, kSlotsQ2, false><<<ntiles, kThreadsQ, sizeof(SmemQ2), s>>>(fp, g, sm, b, st, pool,
+		                                                                              dof_bounds, slice_times);
 	else
-		sample_mbq_kernel<kMaxKeys, kSlotsQ><<<ntiles, kThreadsQ, sizeof(SmemQ), s>>>(fp, g, sm, b, st, dof_bounds,
-		                                                                             slice_times);
+		sample_mbq_kernel<kMaxKeys, kSlotsQ, false><<<ntiles, kThreadsQ, sizeof(SmemQ), s>>>(fp, g, sm, b, st, pool,
+		                                                                                   dof_bounds, slice_times);
 }
 
 void configure_sample_mb_kernels() {
 	static std::mutex mu;
 	static uint64_t configured = 0;
 	if (!first_use_on_device(mu, configured)) return;
-	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemQ));
-	cudaFuncSetAttribute(sample_mbq_kernel<2, kSlotsQ2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	cudaFuncSetAttribute(sample_mbq_kernel<2, kSlotsQ2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemQ2));
+	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     (int)sizeof(SmemQT4));
+	cudaFuncSetAttribute(sample_mbq_kernel<2, kSlotsQ2T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     (int)sizeof(SmemQT2));
 	cudaFuncSetAttribute(sample_mb_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sample_mb_smem(true));
 }
 
