@@ -387,6 +387,7 @@ struct aqh_ctx {
 	bool q8_default = false;  // d_q8 holds the last frame's r g b a display
 	bool dev_motion = false;
 	int dev_max_keys = 0;
+	unsigned long long dev_vertices = 0;  // one past the last Ci / Oi entry any grid uses
 	DevBuf d_queue, d_slices;
 	std::vector<float4> h_dofb;
 	std::vector<float> h_slices;
@@ -718,12 +719,18 @@ void launch_widen3(const float* in, float4* out, size_t n, cudaStream_t s) {
 	const long long blocks = std::min<long long>(((long long)n + 255) / 256, 152LL * 16);
 	widen3_kernel<<<(unsigned)blocks, 256, 0, s>>>(in, out, (long long)n);
 }
-__global__ void any_transparent_kernel(int n, const int32_t* flags, const int32_t* nkeys, int32_t* out) {
+// out: any transparent grid, any moving one, any in camera space, the most
+// keys, and (8 bytes) one past the last vertex of any grid in Ci / Oi.
+__global__ void any_transparent_kernel(int n, const int32_t* flags, const int32_t* nkeys, const int32_t* cu,
+                                       const int32_t* cv, const int64_t* cbase, int32_t* out) {
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i < n && !(flags[i] & AQH_GRID_OPAQUE)) out[0] = 1;
 	if (i < n && nkeys[i] > 1) out[1] = 1;
 	if (i < n && (flags[i] & AQH_GRID_CAMERA)) out[2] = 1;
 	if (i < n) atomicMax(out + 3, nkeys[i]);
+	if (i < n)
+		atomicMax(reinterpret_cast<unsigned long long*>(out + 4),
+		          (unsigned long long)cbase[i] + (unsigned long long)(cu[i] + 1) * (unsigned long long)(cv[i] + 1));
 }
 }  // namespace
 
@@ -835,15 +842,16 @@ aqh_status aqh_submit_grids_device(aqh_ctx* ctx, int ngrids, const int32_t* d_cu
 	AQH_TRY(ctx->d_err.ensure(64), "alloc");
 	AQH_TRY(cudaMemsetAsync(ctx->d_err.p, 0, 64, ctx->stream), "memset");
 	if (ngrids > 0)
-		any_transparent_kernel<<<(ngrids + 255) / 256, 256, 0, ctx->stream>>>(ngrids, d_flags, d_nkeys,
-		                                                                    ctx->d_err.as<int32_t>() + 8);
-	int32_t anyt[4] = {0, 0, 0, 0};
-	AQH_TRY(cudaMemcpyAsync(anyt, ctx->d_err.as<int32_t>() + 8, 16, cudaMemcpyDeviceToHost, ctx->stream), "readback");
+		any_transparent_kernel<<<(ngrids + 255) / 256, 256, 0, ctx->stream>>>(ngrids, d_flags, d_nkeys, d_cu, d_cv,
+		                                                                    d_cbase, ctx->d_err.as<int32_t>() + 8);
+	int32_t anyt[6] = {0, 0, 0, 0, 0, 0};
+	AQH_TRY(cudaMemcpyAsync(anyt, ctx->d_err.as<int32_t>() + 8, sizeof anyt, cudaMemcpyDeviceToHost, ctx->stream), "readback");
 	AQH_TRY(cudaStreamSynchronize(ctx->stream), "sync");
 	ctx->any_transparent = anyt[0] != 0;
 	ctx->dev_motion = anyt[1] != 0;
 	ctx->any_camera = anyt[2] != 0;
 	ctx->dev_max_keys = anyt[3];
+	std::memcpy(&ctx->dev_vertices, anyt + 4, 8);
 	ctx->dev_grids = true;
 	ctx->dev_mps = total_mps;
 	return AQH_OK;
@@ -1074,7 +1082,7 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	// window masks pay off where positions vary across the filter window and
 	// pixels hold few samples (measured: 16 samples, 3x3 pixels)
 	const bool wmask = fp.spp <= 16 && (fp.shiftX > 0 || fp.shiftY > 0) &&
-	                   (2 * fp.shiftX + 1) * (2 * fp.shiftY + 1) <= 32;
+	                   (2 * fp.shiftX + 1) * (2 * fp.shiftY + 1) <= 31;
 	if (wmask) AQH_TRY(ctx->d_wmask.ensure(nstore * sizeof(uint32_t)), "alloc window masks");
 	SampleStore& store = P.store;
 	store = SampleStore{};
@@ -1277,6 +1285,9 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 		AQH_TRY(ctx->d_aovsrc.ensure(nstore * sizeof(int32_t)), "alloc output variable sources");
 		AQH_TRY(ctx->d_aovchan.ensure(ndisp * P.g.naov * sizeof(float)), "alloc output variables");
 		P.store.aovsrc = ctx->d_aovsrc.as<int32_t>();
+		const unsigned long long nv = ctx->host_packed ? ctx->hp.nC
+		                              : ctx->dev_grids ? ctx->dev_vertices : (unsigned long long)ctx->h_verts_c;
+		P.store.aov_vertex = nv <= (unsigned long long)INT32_MAX ? 1 : 0;
 	}
 	return AQH_OK;
 }
@@ -1517,6 +1528,7 @@ aqh_status aqh_render(aqh_ctx* ctx, int sync) {
 	if (!ctx->samples_set) return ctx->fail(AQH_EINVAL, "aqh_set_samples was not called");
 	cudaSetDevice(ctx->device);
 	RenderPlan P;
+	std::memset(static_cast<void*>(&P), 0, sizeof P);  // graphs are found by its bytes, padding included
 	aqh_status st = plan_render(ctx, P);
 	if (st != AQH_OK) return st;
 	ctx->stats.micropolygons = P.nmps;

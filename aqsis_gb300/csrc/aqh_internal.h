@@ -139,6 +139,8 @@ __host__ __device__ inline size_t store_size(long long npix, int spp) {
 	return (size_t)((npix + 31) >> 5) * 32 * (size_t)spp;
 }
 
+constexpr uint32_t kMaskValid = 0x80000000u;  // SampleStore::wmask: the sample holds a hit
+
 // a and b in the store layout above; the debug arrays are pixel-major
 // ([pixel][sample index]).
 struct SampleStore {
@@ -151,12 +153,15 @@ struct SampleStore {
 	                  // depth (midpoint depth filter with a z display), else null
 	uint32_t* wmask;  // per sample (store layout): bit (fy + shiftY) * (2 shiftX + 1) + fx + shiftX set
 	                  // when the sample is inside the filter window of the display pixel at
-	                  // offset (-fx, -fy); null: the filter tests sample positions itself
+	                  // offset (-fx, -fy), and kMaskValid when the sample is valid; null: the
+	                  // filter tests sample positions itself
 	unsigned long long* keys;  // opaque frames: (ordered depth, id + 1) of each sample's occluding
 	                           // hit, pixel-major ([pixel][sample index]), resolved by a separate
 	                           // kernel; null: the sampler resolves in place
 	int32_t* aovsrc;  // micropolygon whose output variables the sample carries after Combine
 	                  // (store layout; -1 none), or null without output variables
+	int aov_vertex;   // every vertex index fits 31 bits: the filter replaces aovsrc's micropolygons by
+	                  // the vertices whose values they carry
 };
 
 // Transparent fragment pool: {depth, micropolygon id bits, u, v} + next link.

@@ -164,7 +164,7 @@ __device__ __forceinline__ void build_record(const FrameParams& fp, const GridsD
 // Final value of one sample: the occluding hit's colour at its (u,v), or the
 // Combine of its transparent fragments; written to the sample store.
 template <bool TRANSP>
-__device__ __forceinline__ void resolve_sample(const FrameParams& fp, const GridsDev& g, const FragPool& pool,
+__device__ __forceinline__ bool resolve_sample(const FrameParams& fp, const GridsDev& g, const FragPool& pool,
                                                const SampleStore& st, long long sidx, long long aidx, float x,
                                                float y, float oz, int w, int head) {
 	float occl[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -207,6 +207,7 @@ __device__ __forceinline__ void resolve_sample(const FrameParams& fp, const Grid
 	if (st.winner) st.winner[sidx] = w;
 	if (st.occlz) st.occlz[sidx] = oz;
 	if (st.nfrag) st.nfrag[sidx] = nf;
+	return valid;
 }
 
 // Phase A: stream the super-tile's grid list from the cursor (lp, r0,
@@ -581,9 +582,10 @@ sample_static_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		const long long pix = (long long)(py - fp.sy0) * fp.sw + (px - fp.sx0);
 		const long long pat = smp.pos_index ? (long long)__ldg(smp.pos_index + pix) : pix;
 		const float2 o = __ldg(smp.pos + pat * spp + si);
-		resolve_sample<TRANSP>(fp, g, pool, st, pix * spp + si, store_index(pix, si, spp), (float)px + o.x, (float)py + o.y,
-		                       sm.soz[s], sm.swin[s], TRANSP ? fhead[s] : -1);
-		if (st.wmask) st.wmask[store_index(pix, si, spp)] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
+		const bool has = resolve_sample<TRANSP>(fp, g, pool, st, pix * spp + si, store_index(pix, si, spp), (float)px + o.x,
+		                                        (float)py + o.y, sm.soz[s], sm.swin[s], TRANSP ? fhead[s] : -1);
+		if (st.wmask) st.wmask[store_index(pix, si, spp)] =
+		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 	}
 	}  // tile loop
 }
@@ -1064,9 +1066,10 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		const long long pix = (long long)(py - fp.sy0) * fp.sw + (px - fp.sx0);
 		const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + si);
 		const unsigned long long kk = sm.key[pl * spp + si];
-		resolve_sample<false>(fp, g, nopool, st, pix * spp + si, store_index(pix, si, spp), (float)px + o.x, (float)py + o.y,
-		                      key_depth(kk), key_winner(kk), -1);
-		if (st.wmask) st.wmask[store_index(pix, si, spp)] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
+		const bool has = resolve_sample<false>(fp, g, nopool, st, pix * spp + si, store_index(pix, si, spp),
+		                                       (float)px + o.x, (float)py + o.y, key_depth(kk), key_winner(kk), -1);
+		if (st.wmask) st.wmask[store_index(pix, si, spp)] =
+		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 	}
 	}  // tile loop
 }
@@ -1086,9 +1089,10 @@ resolve_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, SampleStore st
 	const long long pat = smp.pos_index ? (long long)__ldg(smp.pos_index + pix) : pix;
 	const float2 o = __ldg(smp.pos + pat * fp.spp + si);
 	const unsigned long long kk = st.keys[q0];
-	resolve_sample<false>(fp, g, FragPool{}, st, pix * fp.spp + si, q, (float)px + o.x, (float)py + o.y,
-	                      key_depth(kk), key_winner(kk), -1);
-	if (st.wmask) st.wmask[q] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
+	const bool has = resolve_sample<false>(fp, g, FragPool{}, st, pix * fp.spp + si, q, (float)px + o.x, (float)py + o.y,
+	                                       key_depth(kk), key_winner(kk), -1);
+	if (st.wmask) st.wmask[q] =
+	    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 }
 
 
@@ -1314,9 +1318,10 @@ sample_frag_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sa
 			continue;
 		}
 		const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + si);
-		resolve_sample<true>(fp, g, pool, st, pix * spp + si, store_index(pix, si, spp), (float)px + o.x,
+		const bool has = resolve_sample<true>(fp, g, pool, st, pix * spp + si, store_index(pix, si, spp), (float)px + o.x,
 		                     (float)py + o.y, FLT_MAX, -1, sm.fhead[s]);
-		if (st.wmask) st.wmask[store_index(pix, si, spp)] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
+		if (st.wmask) st.wmask[store_index(pix, si, spp)] =
+		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 	}
 	}  // tile loop
 }
@@ -1339,9 +1344,10 @@ __device__ __forceinline__ void resolve_frag(const FrameParams& fp, const GridsD
 	const int px = fp.sx0 + (int)(pix % fp.sw), py = fp.sy0 + (int)(pix / fp.sw);
 	const long long pat = smp.pos_index ? (long long)__ldg(smp.pos_index + pix) : pix;
 	const float2 o = __ldg(smp.pos + pat * fp.spp + si);
-	resolve_sample<true>(fp, g, pool, st, q, store_index(pix, si, fp.spp), (float)px + o.x, (float)py + o.y,
+	const bool has = resolve_sample<true>(fp, g, pool, st, q, store_index(pix, si, fp.spp), (float)px + o.x, (float)py + o.y,
 	                     OCCL ? st.occlz[q] : FLT_MAX, OCCL ? st.winner[q] : -1, pool.heads[q]);
-	if (st.wmask) st.wmask[store_index(pix, si, fp.spp)] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
+	if (st.wmask) st.wmask[store_index(pix, si, fp.spp)] =
+	    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 }
 
 __global__ void __launch_bounds__(256)

@@ -248,6 +248,12 @@ __device__ __forceinline__ uint32_t window_mask(const FrameParams& fp, int px, i
 	return m;
 }
 
+// The same with bit 31 (kMaskValid) set when the sample holds anything, which
+// spares the filter the sample's opacity record where it only needs that.
+__device__ __forceinline__ uint32_t window_word(const FrameParams& fp, int px, int py, float x, float y, bool has) {
+	return window_mask(fp, px, py, x, y) | (has ? kMaskValid : 0u);
+}
+
 // Grid owning a global micropolygon id: from the id table when there is one,
 // else by binary search over the grids' first ids.
 __device__ __forceinline__ int grid_of(const GridsDev& g, int id) {

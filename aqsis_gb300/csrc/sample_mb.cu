@@ -404,7 +404,7 @@ __device__ __forceinline__ void mb_hit_uv(const FrameParams& fp, const GridsDev&
 }
 
 template <bool TRANSP>
-__device__ __forceinline__ void mb_resolve(const FrameParams& fp, const GridsDev& g, const FragPool& pool,
+__device__ __forceinline__ bool mb_resolve(const FrameParams& fp, const GridsDev& g, const FragPool& pool,
                                            const SampleStore& st, long long sidx, long long aidx, float x, float y,
                                            float stime, float sdx, float sdy, float ozv, int w, int head) {
 	float occl[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -436,6 +436,7 @@ __device__ __forceinline__ void mb_resolve(const FrameParams& fp, const GridsDev
 	if (st.winner) st.winner[sidx] = w;
 	if (st.occlz) st.occlz[sidx] = ozv;
 	if (st.nfrag) st.nfrag[sidx] = nf;
+	return valid;
 }
 
 constexpr int kThreadsM = 512;
@@ -897,12 +898,13 @@ sample_mb_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Samp
 		float x = 0.0f, y = 0.0f, stime = 0.0f, sdx = 0.0f, sdy = 0.0f;
 		int kinv = 0;
 		if (w >= 0) mb_sample_attrs(fp, smp, px, py, j, pix, x, y, stime, sdx, sdy, kinv);
-		mb_resolve<TRANSP>(fp, g, pool, st, pix * spp + j, store_index(pix, j, spp), x, y, stime, sdx, sdy,
+		const bool has = mb_resolve<TRANSP>(fp, g, pool, st, pix * spp + j, store_index(pix, j, spp), x, y, stime, sdx, sdy,
 		                   sm.soz[s], w, TRANSP ? fhead[s] : -1);
 		if (st.wmask) {
 			const long long pp = smp.pos_index ? (long long)__ldg(smp.pos_index + pix) : pix;
 			const float2 o = __ldg(smp.pos + pp * spp + j);
-			st.wmask[store_index(pix, j, spp)] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
+			st.wmask[store_index(pix, j, spp)] =
+			    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 		}
 	}
 }
@@ -1798,9 +1800,10 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 		const unsigned long long kk = sm.key[s];
 		const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
 		const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s]);
-		mb_resolve<TRANSP>(fp, g, pool, st, pix * spp + j, store_index(pix, j, spp), (float)px + o.x, (float)py + o.y,
+		const bool has = mb_resolve<TRANSP>(fp, g, pool, st, pix * spp + j, store_index(pix, j, spp), (float)px + o.x, (float)py + o.y,
 		                   sm.stime[s], d.x, d.y, key_depth_m(kk), key_winner_m(kk), TRANSP ? sm.fhead[s] : -1);
-		if (st.wmask) st.wmask[store_index(pix, j, spp)] = window_mask(fp, px, py, (float)px + o.x, (float)py + o.y);
+		if (st.wmask) st.wmask[store_index(pix, j, spp)] =
+		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 	}
 }
 
