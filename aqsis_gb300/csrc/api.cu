@@ -168,6 +168,15 @@ void set_tiling(FrameParams& fp, int tile_pixels, int supertile_px) {
 	fp.nsty = (fp.nty + fp.st_tiles - 1) / fp.st_tiles;
 }
 
+// Window words pay off where pixels hold few samples (measured: 16 samples, 3x3
+// pixels) and where the rolling filter's windows are 5x5 (480x300, 36 samples:
+// 512 us with words, 795 without).  Their bits hold 31 windows.
+bool window_words(const FrameParams& fp) {
+	const int taps = (2 * fp.shiftX + 1) * (2 * fp.shiftY + 1);
+	const bool roll5 = fp.shiftX == 2 && fp.shiftY == 2 && taps * fp.spp <= kRollTaps;
+	return taps > 1 && taps <= 31 && (fp.spp <= 16 || roll5);
+}
+
 // CqImagePixel::projectToCircle (imagepixel.h:429-436)
 void project_to_circle_h(float x, float y, float& ox, float& oy) {
 	float r;
@@ -379,6 +388,7 @@ struct aqh_ctx {
 	DevBuf d_cu, d_cv, d_nkeys, d_flags, d_tbase, d_pbase, d_cbase, d_mpbase, d_times, d_culled, d_P, d_Ci, d_Oi;
 	DevBuf d_mpcount;
 	DevBuf d_rect, d_minz, d_strips, d_tri, d_stcount, d_stoffset, d_stlist, d_idgrid, d_mpb;
+	DevBuf d_stsorted, d_slack, d_irr, d_redo;  // opaque static frames sampled near to far
 	DevBuf d_sa, d_sb, d_win, d_oz, d_nf, d_hz, d_keys, d_wmask;
 	DevBuf d_frag, d_next, d_fcount, d_foverflow, d_err, d_occl, d_fheads;
 	DevBuf d_ftab, d_chan, d_q8, d_qchan, d_dofb, d_disp, d_dither_req;
@@ -1079,10 +1089,7 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	const size_t nstore = store_size((long long)fp.sw * fp.sh, fp.spp);
 	AQH_TRY(ctx->d_sa.ensure(nstore * sizeof(float4)), "alloc sample store");
 	AQH_TRY(ctx->d_sb.ensure(nstore * sizeof(float4)), "alloc sample store");
-	// window masks pay off where positions vary across the filter window and
-	// pixels hold few samples (measured: 16 samples, 3x3 pixels)
-	const bool wmask = fp.spp <= 16 && (fp.shiftX > 0 || fp.shiftY > 0) &&
-	                   (2 * fp.shiftX + 1) * (2 * fp.shiftY + 1) <= 31;
+	const bool wmask = aqh::window_words(fp);
 	if (wmask) AQH_TRY(ctx->d_wmask.ensure(nstore * sizeof(uint32_t)), "alloc window masks");
 	SampleStore& store = P.store;
 	store = SampleStore{};
@@ -1135,6 +1142,18 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 			AQH_TRY(ctx->d_fheads.ensure(P.nsamp * sizeof(int32_t)), "alloc list heads");
 			pool.heads = ctx->d_fheads.as<int32_t>();
 		}
+	}
+	if (pool.capacity == 0 && !P.mbdof && G > 0) {
+		AQH_TRY(ctx->d_slack.ensure(sizeof(float) * 2 * std::max(G, 1)), "alloc depth slacks");
+		AQH_TRY(ctx->d_irr.ensure(sizeof(uint32_t) * kIrrWords * std::max(G, 1)), "alloc irregular masks");
+		AQH_TRY(ctx->d_redo.ensure(sizeof(int32_t) * (3 + (size_t)kRedoPerTile * fp.ntx * fp.nty)), "alloc redo list");
+		bb.grid_slack = ctx->d_slack.as<float>();
+		bb.grid_nirr = reinterpret_cast<int32_t*>(bb.grid_slack + std::max(G, 1));
+		bb.irregular = ctx->d_irr.as<uint32_t>();
+		bb.redo_next = ctx->d_redo.as<int32_t>();
+		bb.nirr_total = bb.redo_next + 1;
+		bb.nirr_limit = (int32_t)(P.nmps / 8);
+		bb.redo = bb.redo_next + 2;
 	}
 	if (pool.capacity == 0 && !P.mbdof && ctx->host_packed) {
 		// colours still on their way from the host: the sampler hands its
@@ -1315,6 +1334,7 @@ static aqh_status enqueue_frame(aqh_ctx* ctx, RenderPlan& P, bool batched, bool 
 		launch_st_count(fp, P.g, P.bb, s);
 		launch_scan_i32(P.bb.st_count, P.bb.st_offset, P.nst * P.bb.nranges, nullptr, s);
 		launch_st_write(fp, P.g, P.bb, s);
+		if (P.bb.redo) launch_depth_order(fp, P.g, P.bb, s);
 		if (P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, P.bb.mp_stride, s);
 	} else {
 		AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
@@ -1390,7 +1410,12 @@ static aqh_status render_plain(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 	ctx->st_list_cap = std::max<int64_t>(ctx->st_list_cap, ctx->d_stlist.cap / sizeof(int32_t));
 	P.bb.st_list = ctx->d_stlist.as<int32_t>();
 	P.bb.list_capacity = ctx->d_stlist.cap / sizeof(int32_t);
+	if (P.bb.redo) {
+		AQH_TRY(ctx->d_stsorted.ensure(ctx->d_stlist.cap), "alloc tile lists");
+		P.bb.st_sorted = ctx->d_stsorted.as<int32_t>();
+	}
 	if (P.g.ngrids > 0) launch_st_write(fp, P.g, P.bb, s);
+	if (P.bb.redo) launch_depth_order(fp, P.g, P.bb, s);
 	if (P.g.ngrids > 0 && P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, P.bb.mp_stride, s);
 	if (P.g.ngrids <= 0) AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
 	for (int attempt = 0; attempt < 4; ++attempt) {
@@ -1475,6 +1500,10 @@ static aqh_status render_batched(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 	ctx->st_list_cap = ctx->d_stlist.cap / sizeof(int32_t);
 	P.bb.st_list = ctx->d_stlist.as<int32_t>();
 	P.bb.list_capacity = ctx->st_list_cap;
+	if (P.bb.redo) {
+		AQH_TRY(ctx->d_stsorted.ensure(ctx->d_stlist.cap), "alloc tile lists");
+		P.bb.st_sorted = ctx->d_stsorted.as<int32_t>();
+	}
 	// graph key: every kernel argument of the frame
 	std::vector<unsigned char> key(sizeof(RenderPlan) + sizeof(SamplerDev) + sizeof(void*) * 9);
 	unsigned char* k = key.data();

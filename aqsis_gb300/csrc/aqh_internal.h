@@ -192,7 +192,18 @@ struct BinBuffers {
 	int nranges;
 	int range_size;
 	int64_t list_capacity;
+	// opaque static frames sampled near to far (null: in grid order):
+	int32_t* st_sorted;    // st_list with each super-tile's grids by nearest depth, roughly
+	float* grid_slack;     // per grid: no regular micropolygon is hit nearer than its min z less this
+	int32_t* grid_nirr;    // per grid: how many micropolygons are not regular (-1: not known, all of them)
+	uint32_t* irregular;   // per grid kIrrWords words: bit m set when micropolygon m is not regular
+	int32_t* redo;         // [0] count, then the tiles (index) and pixels (~index) to sample in grid order
+	int32_t* redo_next;    // entries of redo handed out
+	int32_t* nirr_total;   // irregular micropolygons of the frame; above nirr_limit all tiles go in
+	int32_t nirr_limit;    // grid order
 };
+constexpr int kIrrWords = 32;     // grids of more micropolygons than bits are not analysed
+constexpr int kRedoPerTile = 8;   // redo entries of a tile at most (more pixels: the whole tile)
 
 // Camera-to-raster matrix of the frame in CqMatrix element order m[row*4 + col].
 struct CamMatrix {
@@ -233,6 +244,8 @@ void launch_project_grids(const GridsDev& g, float4* P, int32_t* flags, const Ca
 void launch_st_count(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cudaStream_t s);
 void launch_scan_i32(const int32_t* in, int32_t* out, int n, int32_t* scratch, cudaStream_t s);
 void launch_st_write(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cudaStream_t s);
+// Fills st_sorted, grid_slack, grid_nirr and irregular, and empties redo.
+void launch_depth_order(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s);
 // `colours_ready`, when given, is an event the first kernel that reads Ci/Oi
 // waits for (on an opaque frame, the resolve after the sampler), with
 // cudaStreamWaitEvent flags `wait_flags` (cudaEventWaitExternal in a capture).
@@ -273,6 +286,9 @@ aqh_status resolve_frame(const aqh_frame_desc& d, FrameParams& fp, std::vector<f
 // (0: 128 pixels).  Neither changes any result.
 void set_tiling(FrameParams& fp, int tile_pixels = 0, int supertile_px = 0);
 void dof_bounds_h(int xs, int ys, std::vector<float4>& out);
+constexpr int kRollTaps = 9 * AQH_MAX_SPP_DEV;  // filter weights the rolling filters hold at most
+// Does the frame keep a window word per sample (SampleStore::wmask)?
+bool window_words(const FrameParams& fp);
 // `q8` (may be null): the frame's r g b a display quantized to 8 bits,
 // written in the same pass (the quantize of quantize_u8 with channels 0 1 2 6).
 void launch_filter(const FrameParams& fp, const SamplerDev& sm, const SampleStore& st, const float* ftab,

@@ -444,6 +444,173 @@ void launch_st_count(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cu
 	st_count_kernel<<<grid, kBlock, 0, s>>>(fp, g.ngrids, b.grid_rect, b.nranges, b.range_size, b.st_count);
 }
 
+// How far below its min z a hit of a micropolygon can lie, or false where no
+// bound is known (an irregular one).
+//
+// The depth of a hit is the bilinear mix of the corner depths at the (u, v) of
+// two Newton steps from the centre C.  With M1 = E + G/2, M2 = F + G/2, area A
+// = M1 x M2 and G = g1 M1 + g2 M2, the first step lands at (x, y) = (u - 1/2, v
+// - 1/2) with M1 x + M2 y = P - C, affine in the sample position P: at the
+// corners x = +-1/2 +- g1/4 and y = +-1/2 +- g2/4, so |x| <= X = 1/2 + |g1|/4
+// and |y| <= Y over the corners' hull, which holds every point the edge tests
+// accept.  The second step's determinant there is A (1 + g2 x + g1 y), also
+// affine, at least A kappa with kappa = 1 - (|g1| + |g2|)/2 - |g1 g2|/2, and
+// its step is -(g1, g2) x y / (det / A).  Hence |u - 1/2| <= U = X + |g1| X Y /
+// kappa, V alike, the weights' absolute values sum to at most W = max(1, 2U)
+// max(1, 2V), the negative ones to (W - 1)/2, and the depth is at least min z -
+// (W - 1)/2 (max z - min z).  Rounding: positions carry 2^-20 of the
+// coordinates into the steps (eta below; a step divides it by kappa), the edge
+// tests accept points up to 2^-10 / kappa < 1/32 of a cell outside for quads
+// with 32 A >= L^2 (L the extent), and the mix itself rounds by 2^-19 W max|z|.
+// Quads with kappa < 0.05 (folded, nearly singular: 1.3% of a grid of unit
+// spacing and +-0.3 jitter), thin ones and anything not finite are irregular.
+__device__ __forceinline__ bool depth_slack(V3f a, V3f b, V3f c, V3f d, float& slack) {
+	const float mnx = fminf(fminf(a.x, b.x), fminf(c.x, d.x)), mxx = fmaxf(fmaxf(a.x, b.x), fmaxf(c.x, d.x));
+	const float mny = fminf(fminf(a.y, b.y), fminf(c.y, d.y)), mxy = fmaxf(fmaxf(a.y, b.y), fmaxf(c.y, d.y));
+	const float mnz = fminf(fminf(a.z, b.z), fminf(c.z, d.z)), mxz = fmaxf(fmaxf(a.z, b.z), fmaxf(c.z, d.z));
+	const float sum = ((a.x + b.x) + (c.x + d.x)) + ((a.y + b.y) + (c.y + d.y)) + ((a.z + b.z) + (c.z + d.z));
+	const float L = (mxx - mnx) + (mxy - mny);
+	const float ex = b.x - a.x, ey = b.y - a.y, fx = c.x - a.x, fy = c.y - a.y;
+	const float gx = (d.x - c.x) - ex, gy = (d.y - c.y) - ey;
+	const float m1x = ex + 0.5f * gx, m1y = ey + 0.5f * gy, m2x = fx + 0.5f * gx, m2y = fy + 0.5f * gy;
+	const float area = fabsf(m1x * m2y - m1y * m2x);
+	if (!(32.0f * area >= L * L && L > 1e-12f && L < 1e6f && fabsf(sum) < 1e30f)) return false;  // NaN too
+	const float ia = 1.0f / area;
+	const float g1 = fabsf(gx * m2y - gy * m2x) * ia, g2 = fabsf(m1x * gy - m1y * gx) * ia;
+	const float cmax = fmaxf(fmaxf(fabsf(mnx), fabsf(mxx)), fmaxf(fabsf(mny), fabsf(mxy)));
+	const float eta = 9.5367432e-7f * (cmax + 4.0f * L) * L * ia;  // 2^-20
+	const float out = 0.03125f + 2.0f * eta;
+	const float X = 0.5f + 0.25f * g1 + out, Y = 0.5f + 0.25f * g2 + out;
+	const float kappa = 1.0f - 0.5f * (g1 + g2) - 0.5f * (g1 * g2) - (g1 + g2) * out - 0.001f;
+	if (!(kappa >= 0.05f)) return false;
+	const float ik = 1.0f / kappa;
+	const float U = X + (g1 * (X * Y) + 8.0f * eta) * ik, V = Y + (g2 * (X * Y) + 8.0f * eta) * ik;
+	const float W = fmaxf(1.0f, 2.0f * U) * fmaxf(1.0f, 2.0f * V);
+	slack = 0.501f * W * (mxz - mnz) + 1.9073486e-6f * W * fmaxf(fabsf(mnz), fabsf(mxz));  // 2^-19
+	return slack < 1e30f;
+}
+
+// WPG warps per grid, 32 micropolygons a warp at a time: the grid's largest
+// slack and which micropolygons are irregular.  Few grids spread theirs over a
+// block (195 grids: 11 us with a warp each, 4 with eight); from some thousands
+// on the warps of other grids fill the SMs and a block each costs more than
+// it gives (200,000 grids: 318 us and 505).
+constexpr int kSlackWarps = 8;
+template <int WPG>
+__global__ void __launch_bounds__(32 * kSlackWarps) grid_slack_kernel(GridsDev g, BinBuffers bb) {
+	__shared__ float most_s[kSlackWarps];
+	__shared__ int nirr_s[kSlackWarps];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wid = warp % WPG;
+	const int gi = blockIdx.x * (kSlackWarps / WPG) + warp / WPG;
+	if (gi >= g.ngrids) return;  // whole warps; with WPG > 1 the block
+	const int cu = __ldg(g.cu + gi), cv = __ldg(g.cv + gi), n = cu * cv;
+	const bool fits = cu <= 1024 && cv <= 1024 && n <= 32 * kIrrWords;
+	const float4* P = g.P + __ldg(g.pbase + gi);
+	float most = 0.0f;
+	int nirr = 0;
+	if (fits)
+		for (int m0 = wid * 32; m0 < n; m0 += 32 * WPG) {
+			const int m = m0 + lane;
+			bool irr = false;
+			if (m < n) {
+				const int iv = m / cu, i = iv * (cu + 1) + (m - iv * cu);
+				float slack = 0.0f;
+				irr = !depth_slack(ld3(P, i), ld3(P, i + 1), ld3(P, i + cu + 1), ld3(P, i + cu + 2), slack);
+				if (!irr) most = fmaxf(most, slack);
+			}
+			const uint32_t w = __ballot_sync(0xffffffffu, irr);
+			if (lane == 0) bb.irregular[(long long)gi * kIrrWords + (m0 >> 5)] = w;
+			nirr += __popc(w);
+		}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+	if (WPG > 1) {
+		static_assert(WPG == 1 || WPG == kSlackWarps, "a block holds one grid's warps");
+		if (lane == 0) {
+			most_s[wid] = most;
+			nirr_s[wid] = nirr;
+		}
+		__syncthreads();
+		if (wid == 0 && lane == 0)
+			for (int w = 1; w < WPG; ++w) {
+				most = fmaxf(most, most_s[w]);
+				nirr += nirr_s[w];
+			}
+	}
+	if (lane != 0 || wid != 0) return;
+	bb.grid_slack[gi] = most;
+	bb.grid_nirr[gi] = fits ? nirr : -1;
+	if (!fits) nirr = n;
+	if (nirr > 0) atomicAdd(bb.nirr_total, nirr);
+}
+
+// One block per super-tile: its grid list by nearest depth, in 1,024 buckets
+// between the list's nearest and farthest (the order within a bucket is left
+// open: no result depends on the order, only how early the near grids come).
+constexpr int kDepthBuckets = 1024;
+__global__ void __launch_bounds__(kDepthBuckets) depth_order_kernel(BinBuffers bb) {
+	__shared__ int count[kDepthBuckets];
+	__shared__ int warp_sum[32];
+	__shared__ uint32_t lo_s, hi_s;
+	const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+	const int beg = bb.st_offset[blockIdx.x * bb.nranges];
+	const int end = (int)min((long long)bb.st_offset[(blockIdx.x + 1) * bb.nranges], (long long)bb.list_capacity);
+	auto depth = [&](int i) -> uint32_t {  // ordered bits of the grid's nearest depth
+		const uint32_t u = __float_as_uint(__ldg(bb.grid_minz + bb.st_list[i]));
+		return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+	};
+	count[t] = 0;
+	if (t == 0) {
+		lo_s = 0xffffffffu;
+		hi_s = 0u;
+	}
+	__syncthreads();
+	uint32_t lo = 0xffffffffu, hi = 0u;
+	for (int i = beg + t; i < end; i += blockDim.x) {
+		const uint32_t k = depth(i);
+		lo = min(lo, k);
+		hi = max(hi, k);
+	}
+	lo = __reduce_min_sync(0xffffffffu, lo);
+	hi = __reduce_max_sync(0xffffffffu, hi);
+	if (lane == 0) {
+		atomicMin(&lo_s, lo);
+		atomicMax(&hi_s, hi);
+	}
+	__syncthreads();
+	lo = lo_s;
+	const float scale = hi_s > lo ? (float)(kDepthBuckets - 1) / (float)(hi_s - lo) : 0.0f;
+	auto bucket = [&](uint32_t k) -> int { return min(kDepthBuckets - 1, (int)((float)(k - lo) * scale)); };
+	for (int i = beg + t; i < end; i += blockDim.x) atomicAdd(&count[bucket(depth(i))], 1);
+	__syncthreads();
+	// exclusive scan of the counts, a bucket per thread
+	const int v = count[t];
+	int x = v;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const int y = __shfl_up_sync(0xffffffffu, x, o);
+		if (lane >= o) x += y;
+	}
+	if (lane == 31) warp_sum[wid] = x;
+	__syncthreads();
+	int pre = 0;
+	for (int w = 0; w < wid; ++w) pre += warp_sum[w];
+	count[t] = beg + pre + x - v;
+	__syncthreads();
+	for (int i = beg + t; i < end; i += blockDim.x)
+		bb.st_sorted[atomicAdd(&count[bucket(depth(i))], 1)] = bb.st_list[i];
+}
+
+void launch_depth_order(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s) {
+	cudaMemsetAsync(b.redo_next, 0, 3 * sizeof(int32_t), s);  // with nirr_total and the redo count
+	if (g.ngrids == 0) return;
+	if (g.ngrids < 4096)
+		grid_slack_kernel<kSlackWarps><<<g.ngrids, 32 * kSlackWarps, 0, s>>>(g, b);
+	else
+		grid_slack_kernel<1><<<(g.ngrids + kSlackWarps - 1) / kSlackWarps, 32 * kSlackWarps, 0, s>>>(g, b);
+	depth_order_kernel<<<fp.nstx * fp.nsty, kDepthBuckets, 0, s>>>(b);
+}
+
 void launch_scan_i32(const int32_t* in, int32_t* out, int n, int32_t*, cudaStream_t s) {
 	scan_i32_kernel<<<1, 1024, 0, s>>>(in, out, n);
 }

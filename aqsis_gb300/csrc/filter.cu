@@ -338,7 +338,6 @@ inline int roll_rows(int cols, int h, int nsm, int per_sm) {
 	while (rows > 1 && (long long)cols * ((h + rows - 1) / rows) < (long long)per_sm * nsm) rows >>= 1;
 	return rows;
 }
-constexpr int kRollTaps = 9 * AQH_MAX_SPP_DEV;  // filter weights a CTA holds at most
 
 // With every sample offset in [0, 1] and half-widths of at least SH + 1/2,
 // every sample of the neighbourhood passes the window test in float: for fx =
@@ -837,11 +836,14 @@ static void launch_filter_sums(const FrameParams& fp, const SamplerDev& sm, cons
 	const int taps = (2 * fp.shiftX + 1) * (2 * fp.shiftY + 1) * fp.spp;
 	const int cols = (w + kRollCols - 1) / kRollCols, rows = roll_rows(cols, h, nsm, 4);
 	if (fp.shiftX == fp.shiftY && (fp.shiftX == 1 || fp.shiftX == 2) && taps <= kRollTaps &&
-	    !(fp.shiftX == 1 && rows < 4 && st.wmask)) {
+	    !(rows < 4 && fp.spp <= 16)) {
 		// 3x3 windows: the rolling window reads each sample three times, not
 		// nine, 5x5 five instead of 25.  Runs of fewer than four rows (images
-		// below about 400x400) lose that: with window words the tile kernel is
-		// faster there (320x240, 4 samples: 12 us against 15)
+		// below about 400x400) lose that where pixels hold few samples
+		// (320x240, 4 samples, 3x3: 12 us on the tile kernel, 15 here; 15
+		// samples, 5x5: 127 and 178), and the tile kernel takes them; with more
+		// samples they gain here too (480x300, 36 samples, 3x3: 332 us against
+		// 129; 211x171, 42 samples, 5x5: 277 against 262)
 		const dim3 rg(cols, (h + rows - 1) / rows);
 		auto go = [&](auto kernel) { kernel<<<rg, kRollThreads, 0, s>>>(fp, sm, st, ftab, channels, q8, rows); };
 		if (fp.shiftX == 1) {

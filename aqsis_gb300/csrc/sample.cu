@@ -210,6 +210,12 @@ __device__ __forceinline__ bool resolve_sample(const FrameParams& fp, const Grid
 	return valid;
 }
 
+// Micropolygon m of grid gid has a bounded depth slack (bin.cu).
+__device__ __forceinline__ bool mp_regular(const BinBuffers& bb, int gid, int m) {
+	return __ldg(bb.grid_nirr + gid) >= 0 &&
+	       !((__ldg(bb.irregular + (long long)gid * kIrrWords + (m >> 5)) >> (m & 31)) & 1u);
+}
+
 // Phase A: stream the super-tile's grid list from the cursor (lp, r0,
 // qtotal) and append the micropolygons that are candidates of the tile to
 // sm.pend, in insertion order, until kSlots are staged or the list ends
@@ -219,11 +225,14 @@ __device__ __forceinline__ bool resolve_sample(const FrameParams& fp, const Grid
 // skipped.  Survivors are compacted with block scans, so the staged order is
 // the insertion order.
 // MAY_CSG: the calling kernel can see CSG grids (the opaque kernel never
-// does: frames with solids always render with fragments).
-template <int kSlots, bool MAY_CSG = true, class Smem>
+// does: frames with solids always render with fragments).  NEAR: the list near
+// to far; a regular micropolygon is behind a depth only with its slack, and of
+// a grid behind every depth the irregular ones are still staged.
+// tw: pixels per row of the tile.
+template <int kSlots, bool MAY_CSG = true, bool NEAR = false, class Smem>
 __device__ __forceinline__ bool stage_candidates(const FrameParams& fp, const GridsDev& g, const BinBuffers& bb,
                                                  Smem& sm, int tpx0, int tpy0, int tpx1, int tpy1, int lend, int& lp,
-                                                 int& r0, int& qtotal, int& npend) {
+                                                 int& r0, int& qtotal, int& npend, int tw) {
 	const int t = threadIdx.x;
 	const int cullable = fp.cullable;
 	while (npend < kSlots) {
@@ -232,22 +241,32 @@ __device__ __forceinline__ bool stage_candidates(const FrameParams& fp, const Gr
 			// grids of the next list chunk that touch the tile, in order
 			const int li = lp + t;
 			int gid = -1, nmp = 0, sub = -1;  // sub: first column, first row, width; -1 = whole grid
-			bool f = false;
+			bool f = false, few = false;  // few: only the irregular ones
 			if (li < lend) {
-				gid = bb.st_list[li];
+				gid = NEAR ? bb.st_sorted[li] : bb.st_list[li];
 				const int4 rc = bb.grid_rect[gid];
 				f = rc.x < rc.y && rc.x < tpx1 && rc.y > tpx0 && rc.z < tpy1 && rc.w > tpy0;
 				if (f && cullable && !(MAY_CSG && csg_grid(g, gid))) {
 					// whole grid behind every sample of the 4x4-pixel blocks it overlaps
 					const int bx0 = (max(rc.x, tpx0) - tpx0) >> 2, bx1 = (min(rc.y, tpx1) - 1 - tpx0) >> 2;
 					const int by0 = (max(rc.z, tpy0) - tpy0) >> 2, by1 = (min(rc.w, tpy1) - 1 - tpy0) >> 2;
-					const int nbx = (fp.tile_w + 3) >> 2;
+					const int nbx = (tw + 3) >> 2;
 					float mx = -FLT_MAX;
 					for (int by = by0; by <= by1; ++by)
 						for (int bx = bx0; bx <= bx1; ++bx) mx = fmaxf(mx, sm.blkmax[by * nbx + bx]);
-					if (__ldg(bb.grid_minz + gid) > mx) f = false;
+					if (NEAR) {
+						const int nirr = __ldg(bb.grid_nirr + gid);
+						if (nirr >= 0 && __ldg(bb.grid_minz + gid) - __ldg(bb.grid_slack + gid) > mx) {
+							f = nirr > 0;
+							few = f;
+							nmp = nirr;
+							sub = -2;
+						}
+					} else if (__ldg(bb.grid_minz + gid) > mx) {
+						f = false;
+					}
 				}
-				if (f) {
+				if (f && !few) {
 					const int cu = __ldg(g.cu + gid), cv = __ldg(g.cv + gid);
 					nmp = cu * cv;
 					if (bb.strips && __ldg(bb.strips + (long long)gid * 64 + 63)) {
@@ -323,6 +342,16 @@ __device__ __forceinline__ bool stage_candidates(const FrameParams& fp, const Gr
 			if (sub >= 0) {
 				const int w = sub >> 16, jv = m / w;
 				m = ((sub >> 8) & 0xff) * cu + jv * cu + (sub & 0xff) + (m - jv * w);
+			} else if (NEAR && sub == -2) {
+				// the m-th irregular micropolygon
+				const uint32_t* irr = bb.irregular + (long long)gid * kIrrWords;
+				int wd = 0;
+				uint32_t w = __ldg(irr);
+				while (m >= __popc(w)) {
+					m -= __popc(w);
+					w = __ldg(irr + ++wd);
+				}
+				m = wd * 32 + (int)__fns(w, 0, m + 1);
 			}
 			const long long pb = __ldg(g.pbase + gid);
 			const int iv = m / cu, iu = m - iv * cu;
@@ -345,8 +374,12 @@ __device__ __forceinline__ bool stage_candidates(const FrameParams& fp, const Gr
 				// early-z for every pixel it visits: behind all their samples' occluding depths
 				float mx = -FLT_MAX;
 				for (int yy = sY; yy < eY; ++yy)
-					for (int xx = sX; xx < eX; ++xx) mx = fmaxf(mx, sm.pixmax[(yy - tpy0) * fp.tile_w + (xx - tpx0)]);
-				if (bminz > mx) active = false;
+					for (int xx = sX; xx < eX; ++xx) mx = fmaxf(mx, sm.pixmax[(yy - tpy0) * tw + (xx - tpx0)]);
+				if (NEAR) {
+					if (bminz - __ldg(bb.grid_slack + gid) > mx && mp_regular(bb, gid, m)) active = false;
+				} else if (bminz > mx) {
+					active = false;
+				}
 			}
 		}
 		int total;
@@ -426,7 +459,7 @@ sample_static_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 	for (;;) {
 		// ---- phase A ----
 		const bool exhausted =
-		    stage_candidates<kSlotsS>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend);
+		    stage_candidates<kSlotsS>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend, fp.tile_w);
 		if (npend == 0) break;
 
 		// ---- build the staged records with every thread busy ----
@@ -692,16 +725,20 @@ __device__ __forceinline__ bool static_hit(const FrameParams& fp, const GridsDev
 	return rec_keeps(g, bb, r.bits, r.id, x, y, u, v);
 }
 
-template <bool PERSIST, int SLOTS, bool MIXED>
+// REDO (with PERSIST): the tiles and single pixels of bb.redo, which the near
+// to far sampler left to the order of insertion.
+template <bool PERSIST, int SLOTS, bool MIXED, bool REDO = false>
 __global__ void __launch_bounds__(kThreadsS, 2)
 sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, SampleStore st, FragPool pool,
                      int* queue, const int* order) {
 	if (MIXED && !*pool.occluders) return;  // sample_frag_kernel renders this frame
+	const bool redo_all = REDO && *bb.nirr_total > bb.nirr_limit;
+	if (REDO && !redo_all && *bb.redo == 0) return;
 	using SmemO = SmemOT<SLOTS, MIXED>;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	SmemO& sm = *reinterpret_cast<SmemO*>(smem_raw);
 	__shared__ int next_tile;
-	const int ntiles = fp.ntx * fp.nty;
+	const int ntiles = REDO && !redo_all ? *bb.redo : fp.ntx * fp.nty;
 	const FragPool nopool{};
 	// MIXED: append the fragments of the lanes with `app` (one per lane, sample
 	// index `at` in pool.heads) from pool slots this warp reserved (a run's rest
@@ -743,26 +780,31 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		__syncthreads();
 		tile = next_tile;
 		if (tile >= ntiles) break;
-		if (order) tile = order[tile];
+		if (REDO) tile = redo_all ? tile : bb.redo[1 + tile];
+		else if (order) tile = order[tile];
 	} else {
 		if (job > 0) break;
 		tile = blockIdx.x;
 	}
-	const int tx = tile % fp.ntx, ty = tile / fp.ntx;
-	const int tpx0 = fp.sx0 + tx * fp.tile_w, tpy0 = fp.sy0 + ty * fp.tile_h;
-	const int tpx1 = min(tpx0 + fp.tile_w, fp.sx0 + fp.sw), tpy1 = min(tpy0 + fp.tile_h, fp.sy0 + fp.sh);
+	// a redo entry below zero is a pixel: a tile of one
+	const bool one = REDO && tile < 0;
+	const int tw = one ? 1 : fp.tile_w, th = one ? 1 : fp.tile_h;
+	const int tx = one ? (~tile % fp.sw) / fp.tile_w : tile % fp.ntx, ty = one ? (~tile / fp.sw) / fp.tile_h : tile / fp.ntx;
+	const int tpx0 = one ? fp.sx0 + ~tile % fp.sw : fp.sx0 + tx * fp.tile_w;
+	const int tpy0 = one ? fp.sy0 + ~tile / fp.sw : fp.sy0 + ty * fp.tile_h;
+	const int tpx1 = min(tpx0 + tw, fp.sx0 + fp.sw), tpy1 = min(tpy0 + th, fp.sy0 + fp.sh);
 	const int st_idx = (ty / fp.st_tiles) * fp.nstx + (tx / fp.st_tiles);
 	const int t = threadIdx.x;
 	const int spp = fp.spp, xs = fp.xs, ys = fp.ys;
 	const uint32_t mxs = div_magic(xs), mys = div_magic(ys);
-	const int tpix = fp.tile_w * fp.tile_h;
+	const int tpix = tw * th;
 	const int tsamp = tpix * spp;
 	const int nflagw = (tsamp + 31) >> 5;
 	const unsigned long long kinit = depth_key(FLT_MAX, -1);
 
 	// MIXED: place of tile sample s of pixel pl in the pixel-major arrays
 	auto sample_at = [&](int pl, int s) -> long long {
-		const int py = tpy0 + pl / fp.tile_w, px = tpx0 + pl % fp.tile_w;
+		const int py = tpy0 + pl / tw, px = tpx0 + pl % tw;
 		return ((long long)(py - fp.sy0) * fp.sw + (px - fp.sx0)) * spp + (s - pl * spp);
 	};
 	for (int i = t; i < tsamp; i += kThreadsS) {
@@ -770,7 +812,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		sm.prev[i] = kinit;
 		if (MIXED) {
 			const int pl = i / spp;
-			if (tpx0 + pl % fp.tile_w < tpx1 && tpy0 + pl / fp.tile_w < tpy1) pool.heads[sample_at(pl, i)] = -1;
+			if (tpx0 + pl % tw < tpx1 && tpy0 + pl / tw < tpy1) pool.heads[sample_at(pl, i)] = -1;
 		}
 	}
 	if (MIXED)
@@ -782,7 +824,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 	if (t < kTilePixMax / 32) sm.dirty[t] = 0u;
 	for (int i = t; i < kTilePixMax; i += kThreadsS) {
 		sm.pixmax[i] = FLT_MAX;
-		const int px = tpx0 + i % fp.tile_w, py = tpy0 + i / fp.tile_w;
+		const int px = tpx0 + i % tw, py = tpy0 + i / tw;
 		int pat = 0;
 		if (i < tpix && px < tpx1 && py < tpy1) {
 			const long long pix = (long long)(py - fp.sy0) * fp.sw + (px - fp.sx0);
@@ -802,7 +844,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 	int lp = lbeg, r0 = 0, qtotal = 0, npend = 0;
 	for (;;) {
 		const bool exhausted =
-		    stage_candidates<SLOTS, false>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend);
+		    stage_candidates<SLOTS, false>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend, tw);
 		if (npend == 0) break;
 
 		// ---- records, and the (candidate, sample) tests RenderMPG_Static makes ----
@@ -836,7 +878,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 				if (occludes)
 					for (int yy = sY; yy < eY; ++yy)
 						for (int xx = sX; xx < eX; ++xx)
-							atomicOr(&sm.mask[(yy - tpy0) * fp.tile_w + (xx - tpx0)][t >> 5], 1u << (t & 31));
+							atomicOr(&sm.mask[(yy - tpy0) * tw + (xx - tpx0)][t >> 5], 1u << (t & 31));
 			}
 		}
 		for (int ph = 0; ph < (MIXED ? 2 : 1); ++ph) {  // occluding candidates, then transparent ones
@@ -888,7 +930,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 				n = q - qd * ys;
 			}
 			const int si = n * xs + m;
-			const int pl = (py - tpy0) * fp.tile_w + (px - tpx0);
+			const int pl = (py - tpy0) * tw + (px - tpx0);
 			const int s = pl * spp + si;
 			if (sm.flag[s >> 5] & (1u << (s & 31))) return;  // replayed in order below
 			const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + si);
@@ -949,7 +991,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 					const int s = wd * 32 + __ffs(fb) - 1;
 					fb &= fb - 1u;
 					const int pl = s / spp, si = s - pl * spp;
-					const int px = tpx0 + pl % fp.tile_w, py = tpy0 + pl / fp.tile_w;
+					const int px = tpx0 + pl % tw, py = tpy0 + pl / tw;
 					if (px >= tpx1 || py >= tpy1) continue;
 					const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + si);
 					const float x = (float)px + o.x, y = (float)py + o.y;
@@ -1018,10 +1060,10 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		if (t < 16 * 16) {
 			// 4x4-pixel block t / 16, one pixel per thread
 			const int b = t >> 4, j = t & 15;
-			const int nbx = (fp.tile_w + 3) >> 2;
+			const int nbx = (tw + 3) >> 2;
 			const int bx = b % nbx, by = b / nbx;
 			const int yy = by * 4 + (j >> 2), xx = bx * 4 + (j & 3);
-			float mx = (yy < fp.tile_h && xx < fp.tile_w) ? sm.pixmax[yy * fp.tile_w + xx] : -FLT_MAX;
+			float mx = (yy < th && xx < tw) ? sm.pixmax[yy * tw + xx] : -FLT_MAX;
 #pragma unroll
 			for (int o = 1; o < 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
 			if (j == 0) sm.blkmax[b] = mx;
@@ -1036,7 +1078,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		// hand the occluding hits to resolve_mixed_kernel, beside the list heads
 		for (int q = t; q < tsamp; q += kThreadsS) {
 			const int pl = q / spp;
-			if (tpx0 + pl % fp.tile_w >= tpx1 || tpy0 + pl / fp.tile_w >= tpy1) continue;
+			if (tpx0 + pl % tw >= tpx1 || tpy0 + pl / tw >= tpy1) continue;
 			const long long at = sample_at(pl, q);
 			st.winner[at] = key_winner(sm.key[q]);
 			st.occlz[at] = key_depth(sm.key[q]);
@@ -1049,7 +1091,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		for (int q = t; q < tsamp; q += kThreadsS) {
 			const int pl = q / spp;
 			const int si = q - pl * spp;
-			const int px = tpx0 + pl % fp.tile_w, py = tpy0 + pl / fp.tile_w;
+			const int px = tpx0 + pl % tw, py = tpy0 + pl / tw;
 			if (px >= tpx1 || py >= tpy1) continue;
 			st.keys[((long long)(py - fp.sy0) * fp.sw + (px - fp.sx0)) * spp + si] = sm.key[pl * spp + si];
 		}
@@ -1061,7 +1103,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 	for (int q = t; q < tsamp; q += kThreadsS) {
 		const int pl = q / spp;
 		const int si = q - pl * spp;
-		const int px = tpx0 + pl % fp.tile_w, py = tpy0 + pl / fp.tile_w;
+		const int px = tpx0 + pl % tw, py = tpy0 + pl / tw;
 		if (px >= tpx1 || py >= tpy1) continue;
 		const long long pix = (long long)(py - fp.sy0) * fp.sw + (px - fp.sx0);
 		const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + si);
@@ -1070,6 +1112,327 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		                                       (float)px + o.x, (float)py + o.y, key_depth(kk), key_winner(kk), -1);
 		if (st.wmask) st.wmask[store_index(pix, si, spp)] =
 		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
+	}
+	}  // tile loop
+}
+
+// ---- opaque frames sampled near to far ----
+//
+// The kernel above visits candidates in insertion order because a hit whose
+// depth D lies below its bound's min z b (rounding, Newton error: an anomalous
+// hit) may be skipped by early-z although D < occlZ, and one not visited could
+// be such a hit.  Neither matters unless depths nearly meet.  Let M be the
+// least (D, id) over all hits of a sample, m the hit.
+//  * If D_m >= b_m, or no other hit has its depth in [M, b_m), the reference
+//    ends with m: when it comes to m, occlZ is FLT_MAX or another hit's depth,
+//    which is at least b_m, so m passes early-z, is stored (occlZ > D_m, or >=
+//    with m first), and nothing later is nearer.
+//  * A regular micropolygon's hits lie no further than its slack below b
+//    (bin.cu), so one with b - slack > z has no hit at or below z.  It can be
+//    skipped when z is the sample's least depth so far, or, where that hit is
+//    anomalous, its b.
+// So candidates come in any order -- near grids first, which hides most of the
+// rest before a vertex of theirs is read -- irregular micropolygons are never
+// skipped, and each sample keeps its least (D, id), a bit for an anomalous hit
+// in the key, and the least depth z2 of all its other tested hits.  At the end
+// a sample whose m is anomalous with z2 < b_m is not decided (a skipped hit
+// within [M, b_m) implies it: what it was skipped for is then a tested hit
+// below b_m), nor is one that met a NaN or zero depth: their pixels, or the
+// tile once there are many, are sampled again by the kernel above (REDO).  So
+// is the whole frame when an eighth of its micropolygons is irregular: testing
+// those behind everything else costs more than the order saves (measured at a
+// quarter, folded quads 25 layers deep: 13.5 against 11.3 ms).
+//
+// Sampling and binning, 16 samples, ordered -> near (ms): 1920x1080 at 25
+// layers 9.1 -> 6.2, at 4 layers 4.5 -> 3.5, at 0.7 1.9 -> 1.8, 640x480 at 0.7
+// 0.36 -> 0.29 (no replays, and 18 KB less shared memory per CTA leave the
+// sample patterns twice the L1): every opaque static frame takes it.  Layers of
+// flat grids at random depths, where rounding makes 40% of the hits anomalous,
+// 15.0 -> 4.1; several layers in exactly one plane, which mostly go in order
+// after all, 19.0 -> 23.4.
+struct RecZ : RecS {
+	float zcull;  // b - slack; -inf: never skipped
+	int pad;      // an odd number of words
+};
+static_assert(sizeof(RecZ) % 8 == 4, "an odd stride spreads neighbouring records over the banks");
+
+struct SmemZ {
+	unsigned long long key[kTileSampMax];   // least hit: (ordered depth, id + 1, anomalous)
+	uint32_t z2[kTileSampMax];              // least depth (ordered) of the other hits
+	RecZ rec[kSlotsO];
+	int2 pend[kSlotsO];
+	int pref[kSlotsO + 1];
+	int rng[kSlotsO][4];
+	int qgrid[kThreadsS];
+	int qcum[kThreadsS + 1];
+	int qsub[kThreadsS];
+	int patidx[kTilePixMax];
+	int warp_tot[32];
+	int first_reject;
+	int qn;
+	float pixmax[kTilePixMax];
+	float blkmax[16];
+	uint32_t dirty[kTilePixMax / 32];
+	uint32_t bad[kTilePixMax / 32];         // pixels to sample again in order
+	int whole;                              // ... or all of them
+};
+
+__device__ __forceinline__ uint32_t ordered_bits(float z) {
+	const uint32_t u = __float_as_uint(z);
+	return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ unsigned long long near_key(float z, int w, bool anomalous) {
+	return ((unsigned long long)ordered_bits(z) << 32) | ((uint32_t)(w + 1) << 1) | (anomalous ? 1u : 0u);
+}
+__device__ __forceinline__ int near_winner(unsigned long long k) { return (int)((uint32_t)k >> 1) - 1; }
+
+// Min z of micropolygon `id` (CalculateBound).
+__device__ __noinline__ float mp_minz(const GridsDev& g, int id) {
+	const int gi = grid_of(g, id);
+	const int cu = __ldg(g.cu + gi);
+	const int m = id - (int)__ldg(g.mpbase + gi), iv = m / cu;
+	const float4* P = g.P + __ldg(g.pbase + gi) + iv * (cu + 1) + (m - iv * cu);
+	return amin(amin(amin(__ldg(P).z, __ldg(P + 1).z), __ldg(P + cu + 2).z), __ldg(P + cu + 1).z);
+}
+
+template <bool PERSIST>
+__global__ void __launch_bounds__(kThreadsS, 2)
+sample_near_kernel(FrameParams fp, const __grid_constant__ GridsDev g, SamplerDev smp, BinBuffers bb, SampleStore st,
+                   int* queue) {
+	if (*bb.nirr_total > bb.nirr_limit) return;
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	SmemZ& sm = *reinterpret_cast<SmemZ*>(smem_raw);
+	__shared__ int next_tile;
+	const int ntiles = fp.ntx * fp.nty;
+	const FragPool nopool{};
+	for (int job = 0;; ++job) {
+	int tile;
+	if (PERSIST) {
+		__syncthreads();
+		if (threadIdx.x == 0) next_tile = atomicAdd(queue, 1);
+		__syncthreads();
+		tile = next_tile;
+		if (tile >= ntiles) break;
+	} else {
+		if (job > 0) break;
+		tile = blockIdx.x;
+	}
+	const int tw = fp.tile_w, th = fp.tile_h;
+	const int tx = tile % fp.ntx, ty = tile / fp.ntx;
+	const int tpx0 = fp.sx0 + tx * tw, tpy0 = fp.sy0 + ty * th;
+	const int tpx1 = min(tpx0 + tw, fp.sx0 + fp.sw), tpy1 = min(tpy0 + th, fp.sy0 + fp.sh);
+	const int st_idx = (ty / fp.st_tiles) * fp.nstx + (tx / fp.st_tiles);
+	const int t = threadIdx.x;
+	const int spp = fp.spp, xs = fp.xs, ys = fp.ys;
+	const uint32_t mxs = div_magic(xs), mys = div_magic(ys);
+	const int tpix = tw * th;
+	const int tsamp = tpix * spp;
+	const unsigned long long kinit = near_key(FLT_MAX, -1, false);
+
+	for (int i = t; i < tsamp; i += kThreadsS) {
+		sm.key[i] = kinit;
+		sm.z2[i] = ordered_bits(FLT_MAX);
+	}
+	if (t < kTilePixMax / 32) {
+		sm.dirty[t] = 0u;
+		sm.bad[t] = 0u;
+	}
+	for (int i = t; i < kTilePixMax; i += kThreadsS) {
+		sm.pixmax[i] = FLT_MAX;
+		const int px = tpx0 + i % tw, py = tpy0 + i / tw;
+		int pat = 0;
+		if (i < tpix && px < tpx1 && py < tpy1) {
+			const long long pix = (long long)(py - fp.sy0) * fp.sw + (px - fp.sx0);
+			pat = smp.pos_index ? (int)__ldg(smp.pos_index + pix) : (int)pix;
+		}
+		sm.patidx[i] = pat;
+	}
+	if (t < 16) sm.blkmax[t] = FLT_MAX;
+	if (t == 0) {
+		sm.qn = 0;
+		sm.qcum[0] = 0;
+		sm.whole = 0;
+	}
+	__syncthreads();
+
+	const int lbeg = bb.st_offset[st_idx * bb.nranges];
+	const int lend = (int)min((long long)bb.st_offset[(st_idx + 1) * bb.nranges], (long long)bb.list_capacity);
+	int lp = lbeg, r0 = 0, qtotal = 0, npend = 0, undecided = 0;
+	for (;;) {
+		const bool exhausted = stage_candidates<kSlotsO, false, true>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0,
+		                                                              qtotal, npend, tw);
+		if (npend == 0) break;
+
+		// records and the (candidate, sample) tests, as in the kernel above
+		int ntests = 0;
+		if (t < npend) {
+			const int2 e = sm.pend[t];
+			RecZ& r = sm.rec[t];
+			build_record(fp, g, e.x, e.y, r);
+			r.zcull = mp_regular(bb, e.x, e.y) ? r.bminz - __ldg(bb.grid_slack + e.x) : -INFINITY;
+			const int sX = max(r.px0, tpx0), eX = min(r.px1, tpx1);
+			const int sY = max(r.py0, tpy0), eY = min(r.py1, tpy1);
+			int cx0 = ((sX == r.px1 - 1) ? r.em : xs) - ((sX == r.px0) ? r.im : 0);
+			int totx = cx0;
+			if (eX - sX > 1) totx += (eX - sX - 2) * xs + ((eX - 1 == r.px1 - 1) ? r.em : xs);
+			int cy0 = ((sY == r.py1 - 1) ? r.en : ys) - ((sY == r.py0) ? r.in_ : 0);
+			int toty = cy0;
+			if (eY - sY > 1) toty += (eY - sY - 2) * ys + ((eY - 1 == r.py1 - 1) ? r.en : ys);
+			totx = max(totx, 0);
+			toty = max(toty, 0);
+			ntests = totx * toty;
+			sm.rng[t][0] = cx0;
+			sm.rng[t][1] = cy0;
+			sm.rng[t][2] = totx;
+			sm.rng[t][3] = (int)div_magic(totx);
+		}
+		int total;
+		const int pre = block_excl_sum(sm.warp_tot, ntests, total);
+		if (t < npend) sm.pref[t] = pre;
+		__syncthreads();
+
+		const int chunk = ((total + kThreadsS - 1) / kThreadsS) * 32;
+		const int pw0 = (t >> 5) * chunk, pw1 = min(total, pw0 + chunk);
+		int cur = 0;
+		for (int p0 = pw0; p0 < pw1; p0 += 32) {
+			const int p = p0 + (t & 31);
+			const int lo = advance_item(sm.pref, npend, cur, min(p, pw1 - 1));
+			cur = __shfl_sync(0xffffffffu, lo, 31);
+			if (p >= pw1) continue;
+			const RecZ& r = sm.rec[lo];
+			const int k = p - sm.pref[lo];
+			const int cx0 = sm.rng[lo][0], cy0 = sm.rng[lo][1], totx = sm.rng[lo][2];
+			const uint32_t mtot = (uint32_t)sm.rng[lo][3];
+			const int sX = max(r.px0, tpx0), sY = max(r.py0, tpy0);
+			const int ky = div_small(k, totx, mtot), kx = k - ky * totx;
+			int px, m, py, n;
+			if (kx < cx0) {
+				px = sX;
+				m = ((sX == r.px0) ? r.im : 0) + kx;
+			} else {
+				const int q = kx - cx0;
+				const int qd = div_small(q, xs, mxs);
+				px = sX + 1 + qd;
+				m = q - qd * xs;
+			}
+			if (ky < cy0) {
+				py = sY;
+				n = ((sY == r.py0) ? r.in_ : 0) + ky;
+			} else {
+				const int q = ky - cy0;
+				const int qd = div_small(q, ys, mys);
+				py = sY + 1 + qd;
+				n = q - qd * ys;
+			}
+			const int si = n * xs + m;
+			const int pl = (py - tpy0) * tw + (px - tpx0);
+			const int s = pl * spp + si;
+			const unsigned long long have = sm.key[s];
+			// behind the sample's least depth (early-z)
+			if (r.zcull > key_depth(have) && !((uint32_t)have & 1u)) continue;
+			const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + si);
+			const float x = (float)px + o.x, y = (float)py + o.y;
+			// CqBound::Contains2D (bound.h:144-151), fContains
+			if ((x < r.bminx || x > r.bmaxx) || (y < r.bminy || y > r.bmaxy)) continue;
+			if ((r.bits & kRecLod) && lod_rejects(fp, g, smp, r.bits >> kRecGridShift, px, py, si)) continue;
+			if (!edges_inside(r.ym, r.xm, r.ex, r.ey, x, y)) continue;
+			float u, v;
+			inv_bilinear(r.ax, r.ay, r.e_x, r.e_y, r.f_x, r.f_y, r.g_x, r.g_y, (r.bits & kRecLinear) != 0, x, y, u,
+			             v);
+			const float D = bilerp1(r.z[0], r.z[1], r.z[2], r.z[3], u, v);
+			if (!rec_keeps(g, bb, r.bits, r.id, x, y, u, v)) continue;
+			if (D != D || D == 0.0f || r.bminz != r.bminz) {
+				// (NaN: the tile, whose culling of whole grids leaves NaN depths out)
+				if (D == 0.0f) atomicOr(&sm.bad[pl >> 5], 1u << (pl & 31));
+				else sm.whole = 1;
+				continue;
+			}
+			const unsigned long long mine = near_key(D, r.id, D < r.bminz);
+			const unsigned long long was = atomicMin(&sm.key[s], mine);
+			// of the two the farther depth is another hit's
+			atomicMin(&sm.z2[s], max((uint32_t)(was >> 32), (uint32_t)(mine >> 32)));
+			if (mine < was) atomicOr(&sm.dirty[pl >> 5], 1u << (pl & 31));
+		}
+		__syncthreads();
+
+		// ---- end of round: what hides candidates at the pixels whose samples
+		// changed (two threads per pixel), then the 4x4-pixel blocks ----
+		for (int u0 = 0; u0 < 2 * tpix; u0 += kThreadsS) {
+			const int u = u0 + t, pp = u >> 1, half = u & 1;
+			const bool act = pp < tpix && (sm.dirty[pp >> 5] & (1u << (pp & 31)));
+			float mx = -FLT_MAX;
+			if (act)
+				for (int k = half; k < spp; k += 2) {
+					const unsigned long long kk = sm.key[pp * spp + k];
+					float z = key_depth(kk);
+					if ((uint32_t)kk & 1u) {
+						z = mp_minz(g, near_winner(kk));
+						if (sm.z2[pp * spp + k] < ordered_bits(z)) atomicOr(&sm.bad[pp >> 5], 1u << (pp & 31));
+					}
+					mx = fmaxf(mx, z);
+				}
+			mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+			if (act && half == 0) sm.pixmax[pp] = mx;
+		}
+		__syncthreads();
+		if (t < kTilePixMax / 32) sm.dirty[t] = 0u;
+		if (t < 16 * 16) {
+			const int b = t >> 4, j = t & 15;
+			const int nbx = (tw + 3) >> 2;
+			const int bx = b % nbx, by = b / nbx;
+			const int yy = by * 4 + (j >> 2), xx = bx * 4 + (j & 3);
+			float mx = (yy < th && xx < tw) ? sm.pixmax[yy * tw + xx] : -FLT_MAX;
+#pragma unroll
+			for (int o = 1; o < 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+			if (j == 0) sm.blkmax[b] = mx;
+		}
+		__syncthreads();
+		npend = 0;
+		// surfaces that coincide: the tile will be sampled in order anyway
+		undecided = sm.whole ? kRedoPerTile + 1 : 0;
+		for (int i = 0; i < kTilePixMax / 32; ++i) undecided += __popc(sm.bad[i]);
+		if (exhausted || undecided > kRedoPerTile) break;
+	}
+	if (undecided > kRedoPerTile) {
+		if (t == 0) bb.redo[1 + atomicAdd(bb.redo, 1)] = tile;
+		if (!PERSIST) break;
+		continue;
+	}
+
+	// ---- the samples, pixel-major: undecided ones are noted; the rest are
+	// resolved, or handed to resolve_opaque_kernel ----
+	for (int q = t; q < tsamp; q += kThreadsS) {
+		const int pl = q / spp;
+		const int si = q - pl * spp;
+		const int px = tpx0 + pl % tw, py = tpy0 + pl / tw;
+		if (px >= tpx1 || py >= tpy1) continue;
+		const long long pix = (long long)(py - fp.sy0) * fp.sw + (px - fp.sx0);
+		const unsigned long long kk = sm.key[q];
+		const float D = key_depth(kk);
+		const int w = near_winner(kk);
+		if (((uint32_t)kk & 1u) && sm.z2[q] < ordered_bits(mp_minz(g, w))) atomicOr(&sm.bad[pl >> 5], 1u << (pl & 31));
+		if (st.keys) {
+			st.keys[pix * spp + si] = depth_key(D, w);
+			continue;
+		}
+		const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + si);
+		const bool has = resolve_sample<false>(fp, g, nopool, st, pix * spp + si, store_index(pix, si, spp),
+		                                       (float)px + o.x, (float)py + o.y, D, w, -1);
+		if (st.wmask)
+			st.wmask[store_index(pix, si, spp)] = window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
+	}
+	__syncthreads();
+	if (t == 0) {
+		int n = 0;
+		for (int i = 0; i < kTilePixMax / 32; ++i) n += __popc(sm.bad[i]);
+		if (n > kRedoPerTile) {
+			bb.redo[1 + atomicAdd(bb.redo, 1)] = tile;
+		} else if (n > 0) {
+			int at = 1 + atomicAdd(bb.redo, n);
+			for (int pl = 0; pl < tpix; ++pl)
+				if ((sm.bad[pl >> 5] >> (pl & 31)) & 1u)
+					bb.redo[at++] = ~((tpy0 + pl / tw - fp.sy0) * fp.sw + (tpx0 + pl % tw - fp.sx0));
+		}
 	}
 	}  // tile loop
 }
@@ -1185,7 +1548,7 @@ sample_frag_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Sa
 	int lp = lbeg, r0 = 0, qtotal = 0, npend = 0;
 	for (;;) {
 		const bool exhausted =
-		    stage_candidates<kSlotsF>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend);
+		    stage_candidates<kSlotsF>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend, fp.tile_w);
 		if (npend == 0) break;
 
 		// records and the (candidate, sample) tests, as on the opaque path
@@ -1453,26 +1816,36 @@ void launch_sample_tiles_q(const FrameParams& fp, const GridsDev& g, const Sampl
 		}
 	}
 	if (mixed) return;
-	if (queue) {
-		if (transp)
+	if (!transp && b.st_sorted) {
+		// near to far, then what that left to the order of insertion
+		if (queue)
+			sample_near_kernel<true><<<nctas, kThreadsS, sizeof(SmemZ), s>>>(fp, g, sm, b, st, queue);
+		else
+			sample_near_kernel<false><<<ntiles, kThreadsS, sizeof(SmemZ), s>>>(fp, g, sm, b, st, nullptr);
+		int dev = 0, nsm = 0;
+		cudaGetDevice(&dev);
+		cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+		sample_opaque_kernel<true, kSlotsO, false, true><<<2 * nsm, kThreadsS, sizeof(SmemO), s>>>(
+		    fp, g, sm, b, st, pool, b.redo_next, nullptr);
+		if (split) {
+			if (colours_ready) cudaStreamWaitEvent(s, colours_ready, wait_flags);
+			launch_resolve_opaque(fp, g, sm, st, s);
+		}
+		return;
+	}
+	if (transp) {
+		if (queue)
 			sample_static_kernel<true, true><<<nctas, kThreadsS, smem_transp, s>>>(fp, g, sm, b, st, pool, queue, order);
 		else
-			sample_opaque_kernel<true, kSlotsO, false><<<nctas, kThreadsS, sizeof(SmemO), s>>>(fp, g, sm, b, st, pool, queue,
-			                                                                                 order);
-		if (split) {
-			if (colours_ready) cudaStreamWaitEvent(s, colours_ready, wait_flags);
-			launch_resolve_opaque(fp, g, sm, st, s);
-		}
-	} else {
-		if (transp)
 			sample_static_kernel<true, false><<<ntiles, kThreadsS, smem_transp, s>>>(fp, g, sm, b, st, pool, nullptr, nullptr);
-		else
-			sample_opaque_kernel<false, kSlotsO, false><<<ntiles, kThreadsS, sizeof(SmemO), s>>>(fp, g, sm, b, st, pool,
-			                                                                                   nullptr, nullptr);
-		if (split) {
-			if (colours_ready) cudaStreamWaitEvent(s, colours_ready, wait_flags);
-			launch_resolve_opaque(fp, g, sm, st, s);
-		}
+		return;
+	}
+	// no depth order (the no-allocation form, frames without grids): in order
+	sample_opaque_kernel<false, kSlotsO, false><<<ntiles, kThreadsS, sizeof(SmemO), s>>>(fp, g, sm, b, st, pool, nullptr,
+	                                                                                   nullptr);
+	if (split) {
+		if (colours_ready) cudaStreamWaitEvent(s, colours_ready, wait_flags);
+		launch_resolve_opaque(fp, g, sm, st, s);
 	}
 }
 
@@ -1494,13 +1867,15 @@ void configure_sample_kernels() {
 	const int smem_transp = (int)(sizeof(SmemS) + sizeof(int32_t) * kTileSampMax);
 	cudaFuncSetAttribute(sample_opaque_kernel<false, kSlotsO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemO));
+	cudaFuncSetAttribute(sample_opaque_kernel<true, kSlotsO, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     (int)sizeof(SmemO));
+	cudaFuncSetAttribute(sample_near_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemZ));
+	cudaFuncSetAttribute(sample_near_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemZ));
 	cudaFuncSetAttribute(sample_opaque_kernel<false, kSlotsMix, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemMix));
 	cudaFuncSetAttribute(sample_opaque_kernel<true, kSlotsMix, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemMix));
 	cudaFuncSetAttribute(sample_static_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_transp);
-	cudaFuncSetAttribute(sample_opaque_kernel<true, kSlotsO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                     (int)sizeof(SmemO));
 	cudaFuncSetAttribute(sample_static_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_transp);
 	cudaFuncSetAttribute(sample_frag_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemF));
 	cudaFuncSetAttribute(sample_frag_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemF));
@@ -1513,7 +1888,7 @@ int sample_static_ctas_per_sm(bool transp) {
 		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sample_static_kernel<true, true>, kThreadsS,
 		                                              sizeof(SmemS) + sizeof(int32_t) * kTileSampMax);
 	else
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sample_opaque_kernel<true, kSlotsO, false>, kThreadsS, sizeof(SmemO));
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sample_near_kernel<true>, kThreadsS, sizeof(SmemZ));
 	return n > 0 ? n : 1;
 }
 

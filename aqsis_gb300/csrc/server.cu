@@ -83,8 +83,10 @@ extern "C" size_t aqh_job_footprint(const aqh_job* j) {
 	int max_keys = 0;
 	for (int i = 0; i < j->ngrids; ++i) max_keys = std::max(max_keys, (int)j->nkeys[i]);
 	const bool moving = fp.use_dof != 0 || max_keys > 1;
+	if (!moving) b += (size_t)j->ngrids * (8 + 4 * aqh::kIrrWords);                      // depth slacks and masks
 	if (moving) b += (size_t)j->micropolygons * (max_keys == 2 ? 32 : 16);               // staging bounds (+ paths)
 	b += nsamp * (32 + 12);                                                              // sample store (+debug)
+	if (aqh::window_words(fp)) b += nsamp * 4;                                           // window words
 	bool transparent = false;
 	for (int i = 0; i < j->ngrids && !transparent; ++i) transparent = !(j->flags[i] & AQH_GRID_OPAQUE);
 	if (transparent) b += std::max<size_t>(1u << 20, nsamp * 2) * 20;                    // fragment pool
