@@ -632,6 +632,9 @@ aqh_status aqh_set_samples(aqh_ctx* ctx, const aqh_samples* s) {
 	m.pos_unit = 1;
 	for (size_t i = 0; i < np && m.pos_unit; ++i)
 		m.pos_unit = s->pos[2 * i] >= 0.0f && s->pos[2 * i] <= 1.0f && s->pos[2 * i + 1] >= 0.0f && s->pos[2 * i + 1] <= 1.0f;
+	m.dof_unit = 1;
+	if (s->dof)
+		for (size_t i = 0; i < 2 * np && m.dof_unit; ++i) m.dof_unit = s->dof[i] >= 0.0f && s->dof[i] <= 1.0f;
 	m.time = s->time ? ctx->s_time.as<float>() : nullptr;
 	m.dof = s->dof ? ctx->s_dof.as<float2>() : nullptr;
 	m.shuffle = s->shuffle ? ctx->s_shuffle.as<int32_t>() : nullptr;
@@ -1143,13 +1146,17 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 			pool.heads = ctx->d_fheads.as<int32_t>();
 		}
 	}
-	if (pool.capacity == 0 && !P.mbdof && G > 0) {
-		AQH_TRY(ctx->d_slack.ensure(sizeof(float) * 2 * std::max(G, 1)), "alloc depth slacks");
-		AQH_TRY(ctx->d_irr.ensure(sizeof(uint32_t) * kIrrWords * std::max(G, 1)), "alloc irregular masks");
+	if (pool.capacity == 0 && G > 0 && P.nmps > 0 && (!P.mbdof || ctx->smp.dof_unit)) {
+		// sampled near to far (the depth bounds under depth of field take lens
+		// offsets inside the lens)
+		if (!P.mbdof) {
+			AQH_TRY(ctx->d_slack.ensure(sizeof(float) * 2 * G), "alloc depth slacks");
+			AQH_TRY(ctx->d_irr.ensure(sizeof(uint32_t) * kIrrWords * G), "alloc irregular masks");
+			bb.grid_slack = ctx->d_slack.as<float>();
+			bb.grid_nirr = reinterpret_cast<int32_t*>(bb.grid_slack + G);
+			bb.irregular = ctx->d_irr.as<uint32_t>();
+		}
 		AQH_TRY(ctx->d_redo.ensure(sizeof(int32_t) * (3 + (size_t)kRedoPerTile * fp.ntx * fp.nty)), "alloc redo list");
-		bb.grid_slack = ctx->d_slack.as<float>();
-		bb.grid_nirr = reinterpret_cast<int32_t*>(bb.grid_slack + std::max(G, 1));
-		bb.irregular = ctx->d_irr.as<uint32_t>();
 		bb.redo_next = ctx->d_redo.as<int32_t>();
 		bb.nirr_total = bb.redo_next + 1;
 		bb.nirr_limit = (int32_t)(P.nmps / 8);
@@ -1335,7 +1342,7 @@ static aqh_status enqueue_frame(aqh_ctx* ctx, RenderPlan& P, bool batched, bool 
 		launch_scan_i32(P.bb.st_count, P.bb.st_offset, P.nst * P.bb.nranges, nullptr, s);
 		launch_st_write(fp, P.g, P.bb, s);
 		if (P.bb.redo) launch_depth_order(fp, P.g, P.bb, s);
-		if (P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, P.bb.mp_stride, s);
+		if (P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb, s);
 	} else {
 		AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
 	}
@@ -1416,7 +1423,7 @@ static aqh_status render_plain(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 	}
 	if (P.g.ngrids > 0) launch_st_write(fp, P.g, P.bb, s);
 	if (P.bb.redo) launch_depth_order(fp, P.g, P.bb, s);
-	if (P.g.ngrids > 0 && P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb.mp_bounds, P.bb.mp_stride, s);
+	if (P.g.ngrids > 0 && P.bb.mp_bounds) launch_mb_stage_bounds(fp, P.g, P.bb, s);
 	if (P.g.ngrids <= 0) AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
 	for (int attempt = 0; attempt < 4; ++attempt) {
 		if (P.pool.capacity > 0) {

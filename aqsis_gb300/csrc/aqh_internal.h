@@ -124,6 +124,7 @@ struct SamplerDev {
 	const uint32_t* shuffle_index;
 	const uint32_t* lod_index;
 	const float* dither;
+	int dof_unit;  // every lens sample is inside [0, 1]^2
 	int pos_unit;  // every position offset is a number in [0, 1] (checked on the host)
 };
 
@@ -192,7 +193,7 @@ struct BinBuffers {
 	int nranges;
 	int range_size;
 	int64_t list_capacity;
-	// opaque static frames sampled near to far (null: in grid order):
+	// opaque frames sampled near to far (null: in grid order; the next three: static ones)
 	int32_t* st_sorted;    // st_list with each super-tile's grids by nearest depth, roughly
 	float* grid_slack;     // per grid: no regular micropolygon is hit nearer than its min z less this
 	int32_t* grid_nirr;    // per grid: how many micropolygons are not regular (-1: not known, all of them)
@@ -250,8 +251,7 @@ void launch_depth_order(const FrameParams& fp, const GridsDev& g, const BinBuffe
 // waits for (on an opaque frame, the resolve after the sampler), with
 // cudaStreamWaitEvent flags `wait_flags` (cudaEventWaitExternal in a capture).
 // Staging bound of every micropolygon of a motion blur / depth of field frame.
-// `stride` 2: each bound is followed by the micropolygon's path (frames of at most two keys).
-void launch_mb_stage_bounds(const FrameParams& fp, const GridsDev& g, int4* out, int stride, cudaStream_t s);
+void launch_mb_stage_bounds(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s);
 void launch_sample_tiles(const FrameParams& fp, const GridsDev& g, const SamplerDev& sm, const BinBuffers& b,
                          SampleStore st, FragPool pool, int32_t* err, cudaStream_t s,
                          cudaEvent_t colours_ready = nullptr, unsigned wait_flags = 0);

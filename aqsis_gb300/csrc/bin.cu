@@ -464,20 +464,27 @@ void launch_st_count(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cu
 // with 32 A >= L^2 (L the extent), and the mix itself rounds by 2^-19 W max|z|.
 // Quads with kappa < 0.05 (folded, nearly singular: 1.3% of a grid of unit
 // spacing and +-0.3 jitter), thin ones and anything not finite are irregular.
-__device__ __forceinline__ bool depth_slack(V3f a, V3f b, V3f c, V3f d, float& slack) {
+//
+// Corners that move (rho > 0) are within rho, per coordinate, of a translate of
+// the given ones: E and F then move by 2 rho, G, M1 and M2 by 4 rho, and the
+// areas by the products' worth of that, against which the bounds are taken.
+__device__ __forceinline__ bool depth_slack(V3f a, V3f b, V3f c, V3f d, float mnz, float mxz, float rho, float far,
+                                            float& slack) {
 	const float mnx = fminf(fminf(a.x, b.x), fminf(c.x, d.x)), mxx = fmaxf(fmaxf(a.x, b.x), fmaxf(c.x, d.x));
 	const float mny = fminf(fminf(a.y, b.y), fminf(c.y, d.y)), mxy = fmaxf(fmaxf(a.y, b.y), fmaxf(c.y, d.y));
-	const float mnz = fminf(fminf(a.z, b.z), fminf(c.z, d.z)), mxz = fmaxf(fmaxf(a.z, b.z), fmaxf(c.z, d.z));
 	const float sum = ((a.x + b.x) + (c.x + d.x)) + ((a.y + b.y) + (c.y + d.y)) + ((a.z + b.z) + (c.z + d.z));
-	const float L = (mxx - mnx) + (mxy - mny);
+	const float L = (mxx - mnx) + (mxy - mny) + 4.0f * rho;
 	const float ex = b.x - a.x, ey = b.y - a.y, fx = c.x - a.x, fy = c.y - a.y;
 	const float gx = (d.x - c.x) - ex, gy = (d.y - c.y) - ey;
 	const float m1x = ex + 0.5f * gx, m1y = ey + 0.5f * gy, m2x = fx + 0.5f * gx, m2y = fy + 0.5f * gy;
-	const float area = fabsf(m1x * m2y - m1y * m2x);
+	const float r4 = 4.0f * rho, r32 = 2.0f * r4 * r4;
+	const float n1 = fabsf(m1x) + fabsf(m1y), n2 = fabsf(m2x) + fabsf(m2y), ng = fabsf(gx) + fabsf(gy);
+	const float area = fabsf(m1x * m2y - m1y * m2x) - (r4 * (n1 + n2) + r32);
 	if (!(32.0f * area >= L * L && L > 1e-12f && L < 1e6f && fabsf(sum) < 1e30f)) return false;  // NaN too
 	const float ia = 1.0f / area;
-	const float g1 = fabsf(gx * m2y - gy * m2x) * ia, g2 = fabsf(m1x * gy - m1y * gx) * ia;
-	const float cmax = fmaxf(fmaxf(fabsf(mnx), fabsf(mxx)), fmaxf(fabsf(mny), fabsf(mxy)));
+	const float g1 = (fabsf(gx * m2y - gy * m2x) + (r4 * (ng + n2) + r32)) * ia;
+	const float g2 = (fabsf(m1x * gy - m1y * gx) + (r4 * (ng + n1) + r32)) * ia;
+	const float cmax = fmaxf(fmaxf(fabsf(mnx), fabsf(mxx)), fmaxf(fabsf(mny), fabsf(mxy))) + far;
 	const float eta = 9.5367432e-7f * (cmax + 4.0f * L) * L * ia;  // 2^-20
 	const float out = 0.03125f + 2.0f * eta;
 	const float X = 0.5f + 0.25f * g1 + out, Y = 0.5f + 0.25f * g2 + out;
@@ -515,7 +522,9 @@ __global__ void __launch_bounds__(32 * kSlackWarps) grid_slack_kernel(GridsDev g
 			if (m < n) {
 				const int iv = m / cu, i = iv * (cu + 1) + (m - iv * cu);
 				float slack = 0.0f;
-				irr = !depth_slack(ld3(P, i), ld3(P, i + 1), ld3(P, i + cu + 1), ld3(P, i + cu + 2), slack);
+				const V3f a = ld3(P, i), b = ld3(P, i + 1), c = ld3(P, i + cu + 1), d = ld3(P, i + cu + 2);
+				irr = !depth_slack(a, b, c, d, fminf(fminf(a.z, b.z), fminf(c.z, d.z)),
+				                   fmaxf(fmaxf(a.z, b.z), fmaxf(c.z, d.z)), 0.0f, 0.0f, slack);
 				if (!irr) most = fmaxf(most, slack);
 			}
 			const uint32_t w = __ballot_sync(0xffffffffu, irr);
@@ -604,7 +613,9 @@ __global__ void __launch_bounds__(kDepthBuckets) depth_order_kernel(BinBuffers b
 void launch_depth_order(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s) {
 	cudaMemsetAsync(b.redo_next, 0, 3 * sizeof(int32_t), s);  // with nirr_total and the redo count
 	if (g.ngrids == 0) return;
-	if (g.ngrids < 4096)
+	if (!b.grid_slack) {
+		// moving frames: the slacks come with the staging bounds
+	} else if (g.ngrids < 4096)
 		grid_slack_kernel<kSlackWarps><<<g.ngrids, 32 * kSlackWarps, 0, s>>>(g, b);
 	else
 		grid_slack_kernel<1><<<(g.ngrids + kSlackWarps - 1) / kSlackWarps, 32 * kSlackWarps, 0, s>>>(g, b);
@@ -621,26 +632,85 @@ void launch_st_write(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cu
 	                                        b.st_list, (long long)b.list_capacity);
 }
 
+// The least depth at which micropolygon m can be hit at any time and lens
+// position, -inf where no bound is known (depth_slack): its corners at a time
+// between two keys are a mix of theirs, so they stay within rho of a translate
+// of key 0's, rho the most any corner's displacement differs from corner 0's
+// plus, under depth of field, the spread of the circles of confusion over its
+// depths (all in front of the eye) times the lens offset, at most 1.
+__device__ __forceinline__ float mb_hit_depth(const FrameParams& fp, const GridsDev& g, int gid, int m,
+                                              const MbStageBound& sb) {
+	const int cu = __ldg(g.cu + gid), nk = __ldg(g.nkeys + gid);
+	const long long nv = (long long)(cu + 1) * (__ldg(g.cv + gid) + 1);
+	const float4* P = g.P + __ldg(g.pbase + gid) + (m / cu) * (cu + 1) + m % cu;
+	const V3f a = ld3(P, 0), b = ld3(P, 1), c = ld3(P, cu + 1), d = ld3(P, cu + 2);
+	float rho = 0.0f, far = 0.0f;
+	for (int k = 1; k < nk; ++k) {
+		const float4* Q = P + k * nv;
+		const V3f a1 = ld3(Q, 0), b1 = ld3(Q, 1), c1 = ld3(Q, cu + 1), d1 = ld3(Q, cu + 2);
+		const float dx = a1.x - a.x, dy = a1.y - a.y;
+		far = fmaxf(far, fmaxf(fabsf(dx), fabsf(dy)));
+		auto off = [&](V3f p, V3f q) { rho = fmaxf(rho, fmaxf(fabsf((q.x - p.x) - dx), fabsf((q.y - p.y) - dy))); };
+		off(b, b1);
+		off(c, c1);
+		off(d, d1);
+		// NaN drops out of the maxima
+		if (!(fabsf((a1.x + a1.y + a1.z) + (b1.x + b1.y + b1.z) + (c1.x + c1.y + c1.z) + (d1.x + d1.y + d1.z)) < 1e30f))
+			return -INFINITY;
+	}
+	if (fp.use_dof) {
+		if (!(sb.mnz > 0.0f && sb.mxz < FLT_MAX)) return -INFINITY;
+		const float2 c1 = coc(sb.mnz, fp.dof_mult, fp.dof_inv_fd, fp.dof_scale_x, fp.dof_scale_y);
+		const float2 c2 = coc(sb.mxz, fp.dof_mult, fp.dof_inv_fd, fp.dof_scale_x, fp.dof_scale_y);
+		const float cx = fmaxf(fabsf(c1.x), fabsf(c2.x)), cy = fmaxf(fabsf(c1.y), fabsf(c2.y));
+		// 1/z - 1/focus keeps its sign over the depths, or the circle passes through 0
+		const bool side = (1.0f / sb.mnz - fp.dof_inv_fd > 0.0f) == (1.0f / sb.mxz - fp.dof_inv_fd > 0.0f);
+		const float lx = side ? fminf(fabsf(c1.x), fabsf(c2.x)) : 0.0f, ly = side ? fminf(fabsf(c1.y), fabsf(c2.y)) : 0.0f;
+		const float spread = fmaxf(cx - lx, cy - ly) + 1e-6f * fmaxf(cx, cy);
+		rho += 1.01f * spread;
+		far += 1.01f * fmaxf(cx, cy);
+		if (!(spread < 1e6f)) return -INFINITY;
+	}
+	// roundings of the corners' mix and shift
+	rho += 4.7683716e-7f * (fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(d.x), fabsf(d.y))) + 2.0f * far);  // 2^-21
+	float slack = 0.0f;
+	if (!depth_slack(a, b, c, d, sb.mnz, sb.mxz, rho, far, slack)) return -INFINITY;
+	return sb.mnz - slack;
+}
+
 // One warp per grid: the staging bound of each of its micropolygons, read by
 // every motion sampling tile the micropolygon may reach instead of its key
 // vertices.  stride 2: each bound is followed by the micropolygon's path.
-__global__ void mb_stage_bounds_kernel(FrameParams fp, GridsDev g, int4* out, int stride) {
+// nirr_total: the frame is sampled near to far, and the bound's least depth is
+// that of its hits (mb_hit_depth) instead of its vertices.
+__global__ void mb_stage_bounds_kernel(FrameParams fp, GridsDev g, int4* out, int stride, int32_t* nirr_total) {
 	const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int lane = threadIdx.x & 31;
 	if (warp >= g.ngrids) return;
 	const int n = __ldg(g.cu + warp) * __ldg(g.cv + warp);
 	int4* o = out + __ldg(g.mpbase + warp) * stride;
+	int nirr = 0;
 	for (int m = lane; m < n; m += 32) {
 		int4 path;
-		o[(long long)m * stride] = pack_stage_bound(mb_stage_bound(fp, g, warp, m, stride == 2 ? &path : nullptr));
+		MbStageBound b = mb_stage_bound(fp, g, warp, m, stride == 2 ? &path : nullptr);
+		if (nirr_total) {
+			b.mnz = mb_hit_depth(fp, g, warp, m, b);
+			if (b.keep && b.mnz == -INFINITY) ++nirr;
+		}
+		o[(long long)m * stride] = pack_stage_bound(b);
 		if (stride == 2) o[(long long)m * 2 + 1] = path;
+	}
+	if (nirr_total) {
+		nirr = __reduce_add_sync(0xffffffffu, nirr);
+		if (lane == 0 && nirr > 0) atomicAdd(nirr_total, nirr);
 	}
 }
 
-void launch_mb_stage_bounds(const FrameParams& fp, const GridsDev& g, int4* out, int stride, cudaStream_t s) {
+void launch_mb_stage_bounds(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s) {
 	if (g.ngrids <= 0) return;
 	const int wpb = kBlock / 32;
-	mb_stage_bounds_kernel<<<(g.ngrids + wpb - 1) / wpb, kBlock, 0, s>>>(fp, g, out, stride);
+	mb_stage_bounds_kernel<<<(g.ngrids + wpb - 1) / wpb, kBlock, 0, s>>>(fp, g, b.mp_bounds, b.mp_stride,
+	                                                                        b.redo ? b.nirr_total : nullptr);
 }
 
 }  // namespace aqh

@@ -39,6 +39,10 @@ __device__ __forceinline__ float mag2diff(V3f a, V3f b) {
 
 constexpr int kDegeneracyMask = 0x8000000;  // micropolygon.h:791
 
+// `m < 1e-8` as the reference's double comparison decides it: 1e-8f is the
+// largest float below 1e-8.  (FP64 issues at 1/64 of the FP32 rate.)
+__device__ __forceinline__ bool coincident(float m) { return m <= 1e-8f; }
+
 // CqMicroPolygon::ComputeVertexOrder (micropolygon.cpp:1207-1284).  v[0..3] are
 // the grid points at index, index+1, index+cu+1, index+cu+2.
 __device__ __forceinline__ int vertex_order(const V3f v[4]) {
@@ -47,14 +51,14 @@ __device__ __forceinline__ int vertex_order(const V3f v[4]) {
 	int codeA = 0, codeB = 1, codeC = 3, codeD = 2;
 	V3f vA = pa, vB = pb, vC = pc;
 	bool degenerate = false;
-	if (mag2diff(pa, pb) < 1e-8) {
+	if (coincident(mag2diff(pa, pb))) {
 		// A--B degenerate: B <- C, C <- D
 		vB = pc; codeB = codeC; vC = pd; codeC = codeD; degenerate = true;
-	} else if (mag2diff(pb, pc) < 1e-8) {
+	} else if (coincident(mag2diff(pb, pc))) {
 		vB = pc; codeB = codeC; vC = pd; codeC = codeD; degenerate = true;
-	} else if (mag2diff(pc, pd) < 1e-8) {
+	} else if (coincident(mag2diff(pc, pd))) {
 		vC = pd; codeC = codeD; degenerate = true;
-	} else if (mag2diff(pd, pa) < 1e-8) {
+	} else if (coincident(mag2diff(pd, pa))) {
 		degenerate = true;  // the reference only drops D here
 	}
 	bool flip = ((vA.x - vB.x) * (vB.y - vC.y)) >= ((vA.y - vB.y) * (vB.x - vC.x));

@@ -1177,15 +1177,6 @@ struct SmemZ {
 	int whole;                              // ... or all of them
 };
 
-__device__ __forceinline__ uint32_t ordered_bits(float z) {
-	const uint32_t u = __float_as_uint(z);
-	return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ unsigned long long near_key(float z, int w, bool anomalous) {
-	return ((unsigned long long)ordered_bits(z) << 32) | ((uint32_t)(w + 1) << 1) | (anomalous ? 1u : 0u);
-}
-__device__ __forceinline__ int near_winner(unsigned long long k) { return (int)((uint32_t)k >> 1) - 1; }
-
 // Min z of micropolygon `id` (CalculateBound).
 __device__ __noinline__ float mp_minz(const GridsDev& g, int id) {
 	const int gi = grid_of(g, id);

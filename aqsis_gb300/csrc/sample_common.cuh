@@ -7,6 +7,22 @@
 
 namespace aqh {
 
+// A sample's nearest hit in the samplers that go near to far: ordered depth
+// bits, micropolygon id + 1 (31 bits), and a bit for an anomalous hit, one
+// below its bound's min z.
+__device__ __forceinline__ uint32_t ordered_bits(float z) {
+	const uint32_t u = __float_as_uint(z);
+	return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float near_depth(unsigned long long k) {
+	const uint32_t o = (uint32_t)(k >> 32);
+	return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+__device__ __forceinline__ unsigned long long near_key(float z, int w, bool anomalous) {
+	return ((unsigned long long)ordered_bits(z) << 32) | ((uint32_t)(w + 1) << 1) | (anomalous ? 1u : 0u);
+}
+__device__ __forceinline__ int near_winner(unsigned long long k) { return (int)((uint32_t)k >> 1) - 1; }
+
 // The level-of-detail test of RenderMPG_Static / RenderMPG_MBOrDof
 // (bucketprocessor.cpp:1182-1190, 1404-1412, 1439-1447): a grid whose
 // LevelOfDetailBounds minimum is >= 0 (the attribute defaults to 0 1,

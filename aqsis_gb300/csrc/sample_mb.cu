@@ -544,9 +544,11 @@ __device__ Bnd sub_bound(const R& r, const float* T, int b) {
 // blocks at the round's start), a micropolygon behind every sample its
 // rectangle covers is not staged: each of its slices' bounds has a min z at
 // or above its own min z less a rounding margin (the slice bounds interpolate
-// key bounds; 1e-6 of the largest |z| is several ulps of it), so every one of
-// its tests would fail early-z.  Returns true when the list is exhausted.
-template <int kSlots, class Smem, int kThreads = kThreadsM>
+// key bounds; 2e-6 of the largest |z| is many ulps of it), so every one of
+// its tests would fail early-z.  NEAR: the list near to far, and the bound's
+// least depth already that of any hit.  Returns true when the list is
+// exhausted.
+template <int kSlots, class Smem, int kThreads = kThreadsM, bool NEAR = false>
 __device__ __forceinline__ bool stage_mb(const FrameParams& fp, const GridsDev& g, const BinBuffers& bb, Smem& sm,
                                          int tpx0, int tpy0, int tpx1, int tpy1, int lend, int& lp, int& r0,
                                          int& qtotal, int& npend, const float* blk = nullptr) {
@@ -559,7 +561,7 @@ __device__ __forceinline__ bool stage_mb(const FrameParams& fp, const GridsDev& 
 			int gid = -1, nmp = 0, sub = -1;  // sub: first column, first row, width; -1 = whole grid
 			bool f = false;
 			if (li < lend) {
-				gid = bb.st_list[li];
+				gid = NEAR ? bb.st_sorted[li] : bb.st_list[li];
 				const int4 rc = bb.grid_rect[gid];
 				f = rc.x < rc.y && rc.x < tpx1 && rc.y > tpx0 && rc.z < tpy1 && rc.w > tpy0;
 			}
@@ -643,8 +645,7 @@ __device__ __forceinline__ bool stage_mb(const FrameParams& fp, const GridsDev& 
 				for (int y = sY; y < eY; ++y)
 					for (int b = (sX - tpx0) >> 2; b <= (eX - 1 - tpx0) >> 2; ++b)
 						zmax = fmaxf(zmax, blk[(y - tpy0) * 4 + b]);
-				const double margin = 1e-6 * (double)fmaxf(fabsf(mnz), fabsf(mxz));
-				if ((double)mnz - margin > (double)zmax) active = false;
+				if (NEAR ? mnz > zmax : mnz - 2e-6f * fmaxf(fabsf(mnz), fabsf(mxz)) > zmax) active = false;
 			}
 		}
 		int total;
@@ -1140,10 +1141,15 @@ struct ItemQ {
 	uint32_t mnpix, mrw;  // ceil(2^32 / npix), ceil(2^32 / rw) (0 for 1): exact quotients of slot indices
 };
 
-template <int NK, int SLOTS, bool TRANSP>
+template <int NK, int SLOTS, bool TRANSP, bool NEAR = false>
 struct SmemQT {
 	unsigned long long key[kTileSampQ];   // occluding hit of each tile sample (depth_key_m)
-	unsigned long long prev[kTileSampQ];  // ... at the start of the round
+	unsigned long long prev[NEAR ? 1 : kTileSampQ];  // ... at the start of the round
+	uint32_t z2[NEAR ? kTileSampQ : 1];   // NEAR: least depth (ordered) of the other hits
+	float zlow[NEAR ? SLOTS : 1];         // least depth of any hit of a candidate
+	uint32_t dirty[kTilePixQ / 32];       // pixels whose samples changed this round
+	uint32_t bad[kTilePixQ / 32];         // pixels whose samples are not decided
+	int whole;                            // the tile is not
 	float stime[kTileSampQ];              // time of each tile sample
 	uint8_t kinv[kTileSampQ];             // lens stratum of each tile sample
 	uint8_t tord[kTileSampQ];             // each pixel's samples by time bin (NaN times last)
@@ -1178,6 +1184,8 @@ struct SmemQT {
 constexpr int kSlotsQ2 = 96, kSlotsQT = 32, kSlotsQ2T = 64;
 using SmemQ = SmemQT<kMaxKeys, kSlotsQ, false>;
 using SmemQ2 = SmemQT<2, kSlotsQ2, false>;
+using SmemQN = SmemQT<kMaxKeys, kSlotsQ, false, true>;
+using SmemQ2N = SmemQT<2, kSlotsQ2, false, true>;
 using SmemQT4 = SmemQT<kMaxKeys, kSlotsQT, true>;
 using SmemQT2 = SmemQT<2, kSlotsQ2T, true>;
 // two CTAs per SM: 228 KB of shared memory less 1 KB reserved per CTA
@@ -1267,16 +1275,49 @@ __device__ __forceinline__ uint32_t quot_magic(int d) {
 // is exact there (the rounding up adds less than r * d / 2^32 / d < 1 / d)
 __device__ __forceinline__ int quot(int r, uint32_t m) { return m == 0u ? r : (int)__umulhi((unsigned)r, m); }
 
-template <int NK, int SLOTS, bool TRANSP>
+// ---- opaque frames near to far (NEAR) ----
+//
+// As sample_near_kernel (sample.cu), whose argument covers (slice, sample)
+// tests as well: a hit is kept when some slice that holds it passes early-z, so
+// its b is the least min z of those slices, and a hit is anomalous when D is
+// below the min z of every one (the key prefers the slice that is not).  No
+// hit of a micropolygon is nearer than its staging bound's least depth
+// (mb_hit_depth).  For an anomalous hit b is bounded by the micropolygon's
+// largest corner depth over all keys; a slice beyond the keys, whose bound is
+// extrapolated past that, leaves its tile undecided.  Undecided tiles, and
+// every tile of a frame with an eighth of its micropolygons irregular, are
+// sampled in order (REDO).  Frame times, ordered -> near (ms): 1920x1080,
+// 36 samples, motion blur + depth of field, 12 layers 156.2 -> 83.2; 640x480,
+// 16 samples, motion blur, 2.5 layers 5.15 -> 4.19; 1280x720 depth of field, 3.3
+// layers 6.00 -> 4.63.  Half of each is the order, the rest the replays that
+// near to far does not need.  With every tile in order after all (grids that
+// turn by 60 degrees, layers in one plane) sampling takes 0.4 to 0.9 of what the
+// ordered kernel took with one thread per replay.
+__device__ __noinline__ float mb_far_corner(const GridsDev& g, int id) {
+	const int gi = grid_of(g, id);
+	const int cu = __ldg(g.cu + gi), nk = __ldg(g.nkeys + gi);
+	const long long nv = (long long)(cu + 1) * (__ldg(g.cv + gi) + 1);
+	const int m = id - (int)__ldg(g.mpbase + gi), iv = m / cu;
+	const float4* P = g.P + __ldg(g.pbase + gi) + iv * (cu + 1) + (m - iv * cu);
+	float z = -FLT_MAX;
+	for (int k = 0; k < nk; ++k, P += nv)
+		z = fmaxf(z, fmaxf(fmaxf(__ldg(P).z, __ldg(P + 1).z), fmaxf(__ldg(P + cu + 1).z, __ldg(P + cu + 2).z)));
+	return z + 1e-6f * fabsf(z);  // above any rounding of a bound between the keys
+}
+
+template <int NK, int SLOTS, bool TRANSP, bool NEAR = false, bool REDO = false>
 __global__ void __launch_bounds__(kThreadsQ, 2)
 sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant__ GridsDev g,
                   const __grid_constant__ SamplerDev smp, const __grid_constant__ BinBuffers bb, SampleStore st,
                   FragPool pool, const float4* dof_bounds, const float* slice_times) {
-	using SmemQ = SmemQT<NK, SLOTS, TRANSP>;
+	using SmemQ = SmemQT<NK, SLOTS, TRANSP, NEAR>;
 	using MbRec = MbRecT<NK>;
+	const bool in_order = (NEAR || REDO) && *bb.nirr_total > bb.nirr_limit;
+	if (NEAR && in_order) return;
+	if (REDO && !in_order && (int)blockIdx.x >= *bb.redo) return;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	SmemQ& sm = *reinterpret_cast<SmemQ*>(smem_raw);
-	const int tile = blockIdx.x;
+	const int tile = REDO && !in_order ? bb.redo[1 + blockIdx.x] : (int)blockIdx.x;
 	const int tx = tile % fp.ntx, ty = tile / fp.ntx;
 	const int tpx0 = fp.sx0 + tx * fp.tile_w, tpy0 = fp.sy0 + ty * fp.tile_h;
 	const int tpx1 = min(tpx0 + fp.tile_w, fp.sx0 + fp.sw), tpy1 = min(tpy0 + fp.tile_h, fp.sy0 + fp.sh);
@@ -1288,7 +1329,7 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 	const int nflagw = (tsamp + 31) >> 5;
 	const bool usingDof = fp.use_dof != 0;
 	const Shutter sh = shutter_of(fp);
-	const unsigned long long kinit = depth_key_m(FLT_MAX, -1);
+	const unsigned long long kinit = NEAR ? near_key(FLT_MAX, -1, false) : depth_key_m(FLT_MAX, -1);
 	// time bins: only moving micropolygons under depth of field use time
 	// windows; the bin of a time is monotone in the time, so a slice's window
 	// [time0, time1] holds no sample outside bins [bin(time0), bin(time1)]
@@ -1305,7 +1346,8 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 	}
 	for (int i = t; i < tsamp; i += kThreadsQ) {
 		sm.key[i] = kinit;
-		sm.prev[i] = kinit;
+		if (NEAR) sm.z2[i] = ordered_bits(FLT_MAX);
+		else sm.prev[i] = kinit;
 		sm.kinv[i] = (uint8_t)(i % spp);
 		if (TRANSP) sm.fhead[i] = -1;
 	}
@@ -1317,6 +1359,11 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 		sm.qn = 0;
 		sm.qcum[0] = 0;
 		sm.any_nan = 0;
+		sm.whole = 0;
+	}
+	if (t < kTilePixQ / 32) {
+		sm.dirty[t] = 0u;
+		sm.bad[t] = 0u;
 	}
 	for (int i = t; i < 16 * 4; i += kThreadsQ) sm.blk[i] = FLT_MAX;
 	__syncthreads();
@@ -1445,11 +1492,11 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 
 	const int lbeg = bb.st_offset[st_idx * bb.nranges];
 	const int lend = (int)min((long long)bb.st_offset[(st_idx + 1) * bb.nranges], (long long)bb.list_capacity);
-	int lp = lbeg, r0 = 0, qtotal = 0, npend = 0;
+	int lp = lbeg, r0 = 0, qtotal = 0, npend = 0, undecided = 0;
 	for (;;) {
 		const bool exhausted =
-			stage_mb<SLOTS, SmemQ, kThreadsQ>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend,
-			                                    sm.blk);
+		    stage_mb<SLOTS, SmemQ, kThreadsQ, NEAR>(fp, g, bb, sm, tpx0, tpy0, tpx1, tpy1, lend, lp, r0, qtotal, npend,
+		                                            sm.blk);
 		if (npend == 0) break;
 
 		// ---- records and (candidate, slice) items ----
@@ -1458,6 +1505,8 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 			const int2 e = sm.pend[t];
 			MbRec& rr = sm.rec[t];
 			build_mb_record(fp, g, e.x, e.y, rr);
+			if (NEAR)
+				sm.zlow[t] = unpack_stage_bound(__ldg(bb.mp_bounds + (__ldg(g.mpbase + e.x) + e.y) * bb.mp_stride)).mnz;
 			int b0 = 0;
 			nitems = 1;
 			if (rr.nkeys > 1) {
@@ -1494,7 +1543,7 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 				for (int py = it.sY; py < it.eY; ++py)
 					for (int px = it.sX; px < it.eX; ++px)
 						zmax = fmaxf(zmax, sm.pxmax[(py - tpy0) * fp.tile_w + (px - tpx0)]);
-				if (it.B.mnz > zmax) continue;
+				if ((NEAR ? sm.zlow[lo] : it.B.mnz) > zmax) continue;
 				const bool moving = r.nkeys > 1;
 				const int rw = it.eX - it.sX, npix = rw * (it.eY - it.sY);
 				int width, wtime, wbase, info = lo | (moving ? 1 << 8 : 0);
@@ -1573,6 +1622,19 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 								app = !(wz[lane] > zk) && !(zk <= D);
 								amb = !app;
 							}
+						} else if (NEAR) {
+							const float b = wz[lane];
+							if (D != D || b != b || (D < b && b > r.bmx[2] + 1e-6f * fabsf(r.bmx[2]))) {
+								sm.whole = 1;
+							} else if (D == 0.0f) {
+								atomicOr(&sm.bad[pl >> 5], 1u << (pl & 31));
+							} else {
+								const unsigned long long mine = near_key(D, r.id, D < b);
+								const unsigned long long was = atomicMin(&sm.key[s], mine);
+								// of the two the farther depth is another hit's
+								atomicMin(&sm.z2[s], max((uint32_t)(was >> 32), (uint32_t)(mine >> 32)));
+								if (mine < was) atomicOr(&sm.dirty[pl >> 5], 1u << (pl & 31));
+							}
 						} else if (!(D >= wz[lane]) || D == 0.0f) {
 							atomicOr(&sm.flag[s >> 5], 1u << (s & 31));
 						} else {
@@ -1629,7 +1691,7 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 					const int px = it.sX + (p - oy * it.rw), py = it.sY + oy;
 					const int pl = (py - tpy0) * fp.tile_w + (px - tpx0);
 					int j = -1;
-					if (it.B.mnz > sm.pxmax[pl]) {
+					if ((NEAR ? sm.zlow[it.info & 0xff] : it.B.mnz) > sm.pxmax[pl]) {
 						// every sample of the pixel is in front of the slice's bound
 					} else if (!(it.info & (1 << 9))) {
 						j = it.wbase + k;
@@ -1646,7 +1708,11 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 						c = it.info & 0xff;
 						const Bnd& B = it.B;
 						bz = B.mnz;
-						pass = !(sm.flag[s >> 5] & (1u << (s & 31)));  // else replayed in order below
+						pass = NEAR || !(sm.flag[s >> 5] & (1u << (s & 31)));  // else replayed in order below
+						if (NEAR) {
+							const unsigned long long have = sm.key[s];
+							pass = !(sm.zlow[c] > near_depth(have) && !((uint32_t)have & 1u));
+						}
 						if (pass && (it.info & (1 << 8))) {
 							const float stime = sm.stime[s];
 							pass = !(stime < it.time0 || stime > it.time1);
@@ -1665,7 +1731,7 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 							pass = !(px < (int)floorf(TB.mnx) || px >= lceil_f(TB.mxx) || py < (int)floorf(TB.mny) ||
 							         py >= lceil_f(TB.mxy)) &&
 							       !((x < TB.mnx || x > TB.mxx) || (y < TB.mny || y > TB.mxy)) &&
-							       !(B.mnz > key_depth_m(sm.prev[s]));
+							       (NEAR || !(B.mnz > key_depth_m(sm.prev[s])));
 						}
 					}
 				}
@@ -1692,6 +1758,26 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 			__syncthreads();
 		}
 		}  // occluding, transparent
+		if (NEAR) {
+			// what hides candidates at the pixels whose samples changed, and
+			// samples not decided so far
+			for (int pl = t; pl < tpix; pl += kThreadsQ) {
+				if (!((sm.dirty[pl >> 5] >> (pl & 31)) & 1u)) continue;
+				float m = -FLT_MAX;
+				for (int j = 0; j < spp; ++j) {
+					const unsigned long long kk = sm.key[pl * spp + j];
+					float z = near_depth(kk);
+					if ((uint32_t)kk & 1u) {
+						z = mb_far_corner(g, near_winner(kk));
+						if (sm.z2[pl * spp + j] < ordered_bits(z)) atomicOr(&sm.bad[pl >> 5], 1u << (pl & 31));
+					}
+					m = fmaxf(m, z);
+				}
+				sm.pxmax[pl] = m;
+			}
+			__syncthreads();
+			if (t < kTilePixQ / 32) sm.dirty[t] = 0u;
+		} else {
 		int anyf = 0;
 		for (int i = t; i < nflagw; i += kThreadsQ) anyf |= (int)(sm.flag[i] != 0u);
 
@@ -1777,6 +1863,7 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 			sm.pxmax[pl] = m;
 		}
 		__syncthreads();
+		}
 		for (int i = t; i < fp.tile_h * 4; i += kThreadsQ) {
 			const int y = i >> 2, x0 = (i & 3) * 4;
 			float m = -FLT_MAX;
@@ -1785,7 +1872,24 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 		}
 		__syncthreads();
 		npend = 0;
-		if (exhausted) break;
+		if (NEAR) {
+			undecided = sm.whole;
+			for (int i = 0; i < kTilePixQ / 32; ++i) undecided |= (int)(sm.bad[i] != 0u);
+		}
+		if (exhausted || undecided) break;
+	}
+	if (NEAR && !undecided) {
+		// hits of later rounds can have left a sample undecided as well
+		bool open = false;
+		for (int q = t; q < tsamp; q += kThreadsQ) {
+			const unsigned long long kk = sm.key[q];
+			if ((uint32_t)kk & 1u) open |= sm.z2[q] < ordered_bits(mb_far_corner(g, near_winner(kk)));
+		}
+		undecided = __syncthreads_or(open);
+	}
+	if (NEAR && undecided) {
+		if (t == 0) bb.redo[1 + atomicAdd(bb.redo, 1)] = tile;
+		return;
 	}
 
 	// ---- resolve, pixel-major (a pixel's samples often share a winner, whose
@@ -1801,7 +1905,8 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 		const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
 		const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s]);
 		const bool has = mb_resolve<TRANSP>(fp, g, pool, st, pix * spp + j, store_index(pix, j, spp), (float)px + o.x, (float)py + o.y,
-		                   sm.stime[s], d.x, d.y, key_depth_m(kk), key_winner_m(kk), TRANSP ? sm.fhead[s] : -1);
+		                   sm.stime[s], d.x, d.y, NEAR ? near_depth(kk) : key_depth_m(kk),
+		                   NEAR ? near_winner(kk) : key_winner_m(kk), TRANSP ? sm.fhead[s] : -1);
 		if (st.wmask) st.wmask[store_index(pix, j, spp)] =
 		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 	}
@@ -1835,10 +1940,17 @@ void launch_sample_mb(const FrameParams& fp, const GridsDev& g, const SamplerDev
 	else if (pool.capacity > 0)
 		sample_mbq_kernel<kMaxKeys, kSlotsQT, true><<<ntiles, kThreadsQ, sizeof(SmemQT4), s>>>(
 		    fp, g, sm, b, st, pool, dof_bounds, slice_times);
-	else if (two)
-		sample_mbq_kernel<2, kSlotsQ2, false><<<ntiles, kThreadsQ, sizeof(SmemQ2), s>>>(fp, g, sm, b, st, pool,
-		                                                                              dof_bounds, slice_times);
-	else
+	else if (b.redo && two) {
+		sample_mbq_kernel<2, kSlotsQ2, false, true><<<ntiles, kThreadsQ, sizeof(SmemQ2N), s>>>(fp, g, sm, b, st, pool,
+		                                                                                    dof_bounds, slice_times);
+		sample_mbq_kernel<2, kSlotsQ2, false, false, true><<<ntiles, kThreadsQ, sizeof(SmemQ2), s>>>(
+		    fp, g, sm, b, st, pool, dof_bounds, slice_times);
+	} else if (b.redo) {
+		sample_mbq_kernel<kMaxKeys, kSlotsQ, false, true><<<ntiles, kThreadsQ, sizeof(SmemQN), s>>>(
+		    fp, g, sm, b, st, pool, dof_bounds, slice_times);
+		sample_mbq_kernel<kMaxKeys, kSlotsQ, false, false, true><<<ntiles, kThreadsQ, sizeof(SmemQ), s>>>(
+		    fp, g, sm, b, st, pool, dof_bounds, slice_times);
+	} else
 		sample_mbq_kernel<kMaxKeys, kSlotsQ, false><<<ntiles, kThreadsQ, sizeof(SmemQ), s>>>(fp, g, sm, b, st, pool,
 		                                                                                   dof_bounds, slice_times);
 }
@@ -1849,7 +1961,13 @@ void configure_sample_mb_kernels() {
 	if (!first_use_on_device(mu, configured)) return;
 	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemQ));
-	cudaFuncSetAttribute(sample_mbq_kernel<2, kSlotsQ2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     (int)sizeof(SmemQN));
+	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ, false, false, true>,
+	                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemQ));
+	cudaFuncSetAttribute(sample_mbq_kernel<2, kSlotsQ2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     (int)sizeof(SmemQ2N));
+	cudaFuncSetAttribute(sample_mbq_kernel<2, kSlotsQ2, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemQ2));
 	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemQT4));

@@ -16,7 +16,8 @@ pytestmark = pytest.mark.gpu
 
 
 def _scene(shutter=(0.0, 1.0), times=(0.0, 1.0), move=(30.0, 4.0), dof=False, z=(1.0, 50.0), shear=0.0, static=0.3,
-           xs=4, ys=4, flat=False, crop=None, transparent=0.0, keys=2, seed=0):
+           xs=4, ys=4, flat=False, crop=None, transparent=0.0, keys=2, grids=160, jitter=0.3,
+           turn=0.0, levels=4, seed=0):
     """Two-key grids over a 72x56 frame, each displaced along `move` turned by a
     random angle, key 1 sheared by `shear`; a share `static` has one key, a share
     `transparent` lets what lies behind it through."""
@@ -25,16 +26,19 @@ def _scene(shutter=(0.0, 1.0), times=(0.0, 1.0), move=(30.0, 4.0), dof=False, z=
     if dof:
         fr.fstop, fr.focal_length, fr.focal_distance, fr.dof_scale = 2.8, 0.4, 20.0, (40.0, 40.0)
     parts = []
-    for i in range(160):
+    for i in range(grids):
         n = int(rng.integers(1, 9))
-        g = S.regular_grids(1, 72, 56, rng, n=n, zrange=z, slope=0.0 if flat else 0.02, motion=1.0,
+        g = S.regular_grids(1, 72, 56, rng, n=n, zrange=z, slope=0.0 if flat else 0.02, motion=1.0, jitter=jitter,
                             origin_margin=10.0)
         P = g.P.reshape(2, -1, 4)
         a = rng.uniform(0, 2 * np.pi)
         d = np.array([np.cos(a) * move[0] - np.sin(a) * move[1], np.sin(a) * move[0] + np.cos(a) * move[1]])
         P[1, :, :2] = P[0, :, :2] + d + shear * (P[0, :, :2] - P[0, 0, :2])[:, ::-1]
+        if turn:
+            c, sn = np.cos(turn), np.sin(turn)
+            P[1, :, :2] = P[1, 0, :2] + (P[1, :, :2] - P[1, 0, :2]) @ np.array([[c, -sn], [sn, c]], np.float32)
         if flat:
-            P[:, :, 2] = float(rng.integers(2, 5))   # coplanar layers: depths tie and round below their bounds
+            P[:, :, 2] = float(rng.integers(2, 1 + levels))   # coplanar layers: depths tie and round below their bounds
         if rng.random() < transparent:
             g.Oi[:, :3] = rng.uniform(0.1, 1.05, (len(g.Oi), 3))   # some corners opaque
             g.flags &= ~np.int32(S.GRID_OPAQUE)
@@ -60,6 +64,12 @@ CASES = {
     "dof": dict(dof=True, move=(12.0, 1.0)), "dof_depth_reaches_zero": dict(dof=True, z=(-0.05, 0.05), move=(8.0, 0.0)),
     "samples_1x1": dict(xs=1, ys=1), "samples_16x16": dict(xs=16, ys=16, move=(10.0, 0.0)), "samples_5x3": dict(xs=5, ys=3),
     "crop": dict(crop=(13, 61, 9, 40)), "flat": dict(flat=True), "flat_dof": dict(flat=True, dof=True, move=(6.0, 0.0)),
+    "deep": dict(grids=900, move=(5.0, 1.0)), "deep_dof": dict(grids=900, dof=True, move=(4.0, 0.0)),
+    "deep_static_dof": dict(grids=900, dof=True, static=1.0), "deep_folded": dict(grids=700, jitter=0.9, move=(3.0, 0.0)),
+    "deep_turning": dict(grids=700, turn=1.2, move=(6.0, 0.0)), "deep_4_keys": dict(grids=700, keys=4, move=(8.0, 0.0)),
+    "deep_flat": dict(grids=700, flat=True, levels=60, move=(3.0, 0.0)),
+    "deep_near_eye": dict(grids=700, dof=True, z=(0.05, 2.0), move=(2.0, 0.0)),
+    "deep_beyond_keys": dict(grids=700, times=(0.4, 0.5), move=(4.0, 0.0)),
     "transparent": dict(transparent=0.5, move=(12.0, 2.0)), "transparent_all": dict(transparent=1.0, move=(6.0, 0.0)),
     "transparent_dof": dict(transparent=0.5, dof=True, move=(12.0, 2.0)),
     "transparent_flat": dict(transparent=0.5, flat=True, move=(9.0, 0.0)),
