@@ -100,3 +100,24 @@ def test_deep_frame_with_nan_depths(aqh_lib):
     assert np.array_equal(a["winner"], b["winner"])
     assert np.array_equal(a["occlz"].view(np.uint32), b["occlz"].view(np.uint32))
     assert (a["winner"] != clean["winner"]).mean() < 0.01
+
+
+def test_list_entries_are_reported(aqh_lib):
+    """A plain frame that did not wait for binning reports its list entries on
+    request, as the batched form does; each of two frames its own."""
+    a, b = _scene(seed=1), _scene(seed=2, w=300, h=200, layers=1.0)
+    want, got = [], []
+    for batched, out in ((True, want), (False, got)):
+        h = aqh_lib.Hider(0)
+        try:
+            h.set_mode(batched)
+            for sc in (a, b):
+                h.frame_begin(sc.frame)
+                h.set_samples(sc.samples)
+                h.submit_grids_host(sc.grids)
+                h.render(sync=batched)
+                out.append(h.stats()["tile_grid_pairs"])
+                h.synchronize()
+        finally:
+            h.close()
+    assert want == got and min(want) > 0 and want[0] != want[1]
