@@ -454,16 +454,19 @@ void launch_st_count(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cu
 // corners x = +-1/2 +- g1/4 and y = +-1/2 +- g2/4, so |x| <= X = 1/2 + |g1|/4
 // and |y| <= Y over the corners' hull, which holds every point the edge tests
 // accept.  The second step's determinant there is A (1 + g2 x + g1 y), also
-// affine, at least A kappa with kappa = 1 - (|g1| + |g2|)/2 - |g1 g2|/2, and
-// its step is -(g1, g2) x y / (det / A).  Hence |u - 1/2| <= U = X + |g1| X Y /
+// affine, so at least A kappa with kappa its least value at the corners, 1 +-
+// (g1 + g2)/2 + g1 g2/2 and 1 +- (g1 - g2)/2 - g1 g2/2, and its step is -(g1,
+// g2) x y / (det / A).  Hence |u - 1/2| <= U = X + |g1| X Y /
 // kappa, V alike, the weights' absolute values sum to at most W = max(1, 2U)
 // max(1, 2V), the negative ones to (W - 1)/2, and the depth is at least min z -
 // (W - 1)/2 (max z - min z).  Rounding: positions carry 2^-20 of the
 // coordinates into the steps (eta below; a step divides it by kappa), the edge
-// tests accept points up to 2^-10 / kappa < 1/32 of a cell outside for quads
-// with 32 A >= L^2 (L the extent), and the mix itself rounds by 2^-19 W max|z|.
-// Quads with kappa < 0.05 (folded, nearly singular: 1.3% of a grid of unit
-// spacing and +-0.3 jitter), thin ones and anything not finite are irregular.
+// tests accept points up to 2^-10 / c < 1/32 of a cell outside for quads with
+// 32 A >= L^2 (L the extent) whose corners turn by at least c A, c = 1 - (|g1| +
+// |g2|)/2 >= 0.05, and the mix itself rounds by 2^-19 W max|z|.  Quads with
+// kappa < 0.05 or c < 0.05 (folded, nearly singular: one in 2,000 of a grid of
+// unit spacing and +-0.3 jitter), thin ones and anything not finite are
+// irregular.
 //
 // Corners that move (rho > 0) are within rho, per coordinate, of a translate of
 // the given ones: E and F then move by 2 rho, G, M1 and M2 by 4 rho, and the
@@ -479,17 +482,28 @@ __device__ __forceinline__ bool depth_slack(V3f a, V3f b, V3f c, V3f d, float mn
 	const float m1x = ex + 0.5f * gx, m1y = ey + 0.5f * gy, m2x = fx + 0.5f * gx, m2y = fy + 0.5f * gy;
 	const float r4 = 4.0f * rho, r32 = 2.0f * r4 * r4;
 	const float n1 = fabsf(m1x) + fabsf(m1y), n2 = fabsf(m2x) + fabsf(m2y), ng = fabsf(gx) + fabsf(gy);
-	const float area = fabsf(m1x * m2y - m1y * m2x) - (r4 * (n1 + n2) + r32);
+	const float cross = m1x * m2y - m1y * m2x;
+	const float area = fabsf(cross) - (r4 * (n1 + n2) + r32);
 	if (!(32.0f * area >= L * L && L > 1e-12f && L < 1e6f && fabsf(sum) < 1e30f)) return false;  // NaN too
 	const float ia = 1.0f / area;
+	// g1 and g2 of the given corners, and their magnitudes with the movement
+	const float s1 = (gx * m2y - gy * m2x) / cross, s2 = (m1x * gy - m1y * gx) / cross;
 	const float g1 = (fabsf(gx * m2y - gy * m2x) + (r4 * (ng + n2) + r32)) * ia;
 	const float g2 = (fabsf(m1x * gy - m1y * gx) + (r4 * (ng + n1) + r32)) * ia;
+	const float turn = 1.0f - 0.5f * (g1 + g2);
 	const float cmax = fmaxf(fmaxf(fabsf(mnx), fabsf(mxx)), fmaxf(fabsf(mny), fabsf(mxy))) + far;
 	const float eta = 9.5367432e-7f * (cmax + 4.0f * L) * L * ia;  // 2^-20
 	const float out = 0.03125f + 2.0f * eta;
 	const float X = 0.5f + 0.25f * g1 + out, Y = 0.5f + 0.25f * g2 + out;
-	const float kappa = 1.0f - 0.5f * (g1 + g2) - 0.5f * (g1 * g2) - (g1 + g2) * out - 0.001f;
-	if (!(kappa >= 0.05f)) return false;
+	// the movement changes s1 by at most t1 = r (1 + |s1|), r the areas' relative
+	// change, and the corner values by at most (t1 + t2)(1 + max g)/2 + t1 t2/2
+	const float t1 = g1 - fabsf(s1) + 2.0f * (fabsf(cross) - area) * ia * fabsf(s1);
+	const float t2 = g2 - fabsf(s2) + 2.0f * (fabsf(cross) - area) * ia * fabsf(s2);
+	const float moved = 0.5f * (t1 + t2) * (1.0f + fmaxf(g1, g2)) + 0.5f * (t1 * t2);
+	const float h = 0.5f * (s1 * s2);
+	const float kappa = 1.0f + fminf(h - 0.5f * fabsf(s1 + s2), -h - 0.5f * fabsf(s1 - s2)) - moved -
+	                    (g1 + g2) * out - 0.001f;
+	if (!(kappa >= 0.05f && turn >= 0.05f)) return false;
 	const float ik = 1.0f / kappa;
 	const float U = X + (g1 * (X * Y) + 8.0f * eta) * ik, V = Y + (g2 * (X * Y) + 8.0f * eta) * ik;
 	const float W = fmaxf(1.0f, 2.0f * U) * fmaxf(1.0f, 2.0f * V);

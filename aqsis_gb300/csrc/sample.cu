@@ -1144,7 +1144,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 // quarter, folded quads 25 layers deep: 13.5 against 11.3 ms).
 //
 // Sampling and binning, 16 samples, ordered -> near (ms): 1920x1080 at 25
-// layers 9.1 -> 6.2, at 4 layers 4.5 -> 3.5, at 0.7 1.9 -> 1.8, 640x480 at 0.7
+// layers 9.1 -> 5.7, at 4 layers 4.5 -> 3.4, at 0.7 1.9 -> 1.8, 640x480 at 0.7
 // 0.36 -> 0.29 (no replays, and 18 KB less shared memory per CTA leave the
 // sample patterns twice the L1): every opaque static frame takes it.  Layers of
 // flat grids at random depths, where rounding makes 40% of the hits anomalous,

@@ -1287,9 +1287,9 @@ __device__ __forceinline__ int quot(int r, uint32_t m) { return m == 0u ? r : (i
 // extrapolated past that, leaves its tile undecided.  Undecided tiles, and
 // every tile of a frame with an eighth of its micropolygons irregular, are
 // sampled in order (REDO).  Frame times, ordered -> near (ms): 1920x1080,
-// 36 samples, motion blur + depth of field, 12 layers 156.2 -> 83.2; 640x480,
-// 16 samples, motion blur, 2.5 layers 5.15 -> 4.19; 1280x720 depth of field, 3.3
-// layers 6.00 -> 4.63.  Half of each is the order, the rest the replays that
+// 36 samples, motion blur + depth of field, 12 layers 156.2 -> 75.3; 640x480,
+// 16 samples, motion blur, 2.5 layers 5.15 -> 4.07; 1280x720 depth of field, 3.3
+// layers 6.00 -> 4.43.  Half of each is the order, the rest the replays that
 // near to far does not need.  With every tile in order after all (grids that
 // turn by 60 degrees, layers in one plane) sampling takes 0.4 to 0.9 of what the
 // ordered kernel took with one thread per replay.
