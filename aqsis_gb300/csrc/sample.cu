@@ -8,25 +8,29 @@
 //
 // Layout.  One CTA (16 warps) owns a tile of the sample region holding at
 // most 4096 samples (16x16 pixels at 16 samples per pixel).  It walks its
-// super-tile's grid list in submission order and expands the grids touching
-// the tile into micropolygons, kSlotsS at a time:
+// super-tile's grid list and expands the grids touching the tile into
+// micropolygons, a round of some hundred at a time:
 //   phase A: one micropolygon per thread tests bound, crop cull and a
-//     tile-wide early-z; survivors are compacted in insertion order, then
-//     every thread builds one shared-memory record (vertex order, edge and
-//     inverse-bilinear coefficients, pixel and sub-sample ranges) and sets a
-//     bit per covered pixel in that pixel's candidate mask;
-//   phase B: a warp takes 32 consecutive samples of the tile, one per lane,
-//     and walks the union of their pixels' masks in ascending slot order --
-//     the insertion order -- with warp-uniform control flow: records are
-//     shared-memory broadcasts, a candidate behind all 32 samples' occluding
-//     depths is skipped by the whole warp, and each lane runs the reference's
-//     per-sample sequence (sub-sample range, inclusive bound test, early-z,
-//     edge tests, inverse bilinear, depth, store).
-// Because each sample is owned by one lane that visits its candidates in
-// insertion order, the reference's order-dependent early-z and its "first of
-// equal depths wins" rule hold exactly.  Colours are resolved once per sample at the
-// end (the reference interpolates them at store time; the values are the
-// same because they depend only on the winning micropolygon and (u,v)).
+//     tile-wide early-z; survivors are compacted in list order, then every
+//     thread builds one shared-memory record (vertex order, edge and
+//     inverse-bilinear coefficients, pixel and sub-sample ranges);
+//   phase B: the hit tests, in one of these forms:
+//     sample_near_kernel: opaque frames, grids near to far; pixels whose
+//       result could depend on the order go to a list;
+//     sample_opaque_kernel: in insertion order, (micropolygon, sample) pairs
+//       in parallel; that list, frames without a depth order, and (MIXED)
+//       transparent frames with occluders;
+//     sample_frag_kernel: frames in which every hit is a fragment;
+//     sample_static_kernel: CSG solids, midpoint depths and samples that may
+//       not be culled: a warp takes 32 samples, one per lane, and walks the
+//       union of their pixels' candidate masks in insertion order, each lane
+//       running the reference's per-sample sequence (sub-sample range,
+//       inclusive bound test, early-z, edge tests, inverse bilinear, depth,
+//       store).
+// Each section says why its form keeps the reference's order-dependent early-z
+// and its "first of equal depths wins" rule.  Colours are resolved once per
+// sample at the end (the reference interpolates them at store time; the values
+// are the same because they depend only on the winning micropolygon and (u,v)).
 #include "aqh_internal.h"
 #include "hider_device.cuh"
 #include "sample_common.cuh"

@@ -147,18 +147,20 @@ WORKLOADS = {
 }
 
 
-KERNELS = {"opaque": "sample_opaque_kernel", "transparent": "sample_frag_kernel + resolve_frag_kernel", "mbdof": "sample_mbq_kernel",
-           "spheres": "sample_opaque_kernel"}
+KERNELS = {"opaque": "sample_near_kernel", "transparent": "sample_frag_kernel + resolve_frag_kernel", "mbdof": "sample_mbq_kernel",
+           "spheres": "sample_near_kernel"}
 # kernels one batched frame launches: id table, grid rects, super-tile count,
 # scan, super-tile write (binning); the sampler(s); the filter, which also
-# quantizes the frame's 8-bit display.  The transparent frame launches the
-# occluder scan, both static samplers (one returns at once) and the Combine
-# kernel of fragment-only frames (which returns at once when the ordered
-# sampler ran); the motion frame the staging-bounds kernel before its sampler.
-LAUNCHES = {"opaque": 7, "transparent": 10, "mbdof": 8, "spheres": 8}  # spheres: + the projection
+# quantizes the frame's 8-bit display.  Opaque frames add the depth slacks and
+# the near-to-far order to binning, and the ordered sampler of what the
+# near-to-far one left; in motion frames the staging-bounds kernel finds the
+# slacks.  The transparent frame launches the occluder scan, the
+# fragment-only sampler and its Combine kernel, and the sampler of frames with
+# occluders and its own (one pair of the two returns at once).
+LAUNCHES = {"opaque": 10, "transparent": 11, "mbdof": 10, "spheres": 11}  # spheres: + the projection
 L2_BYTES = 129 << 20
 # measured DRAM bytes per micropolygon of the sampler launch (ncu, 0.35 scale)
-TRAFFIC_PER_MP = {"opaque": (98.411520e6 + 142.133760e6) / 6_272_000}
+TRAFFIC_PER_MP = {"opaque": (85.522432e6 + 142.624768e6) / 6_272_000}
 
 
 def make_scene(args):
@@ -542,7 +544,7 @@ def run_gpu(args):
     alg_bytes = g.nbytes_algorithmic()  # P + Ci + Oi float4 per vertex, read once
     # DRAM bytes (read + write) of one sampler launch from an ncu capture of the
     # same kernel on a smaller frame of the same stream, scaled by micropolygons
-    # (profiles/sample_opaque_kernel_opaque_stream_scale035.md); None where no
+    # (profiles/sample_near_kernel_opaque_stream_scale035.md); None where no
     # capture of that kernel exists
     traffic = TRAFFIC_PER_MP[args.workload] * mps if TRAFFIC_PER_MP.get(args.workload) else None
     ms_sample = r["stage"]["sample"]
