@@ -759,9 +759,22 @@ __global__ void any_transparent_kernel(int n, const int32_t* flags, const int32_
 	if (i < n && nkeys[i] > 1) out[1] = 1;
 	if (i < n && (flags[i] & AQH_GRID_CAMERA)) out[2] = 1;
 	if (i < n) atomicMax(out + 3, nkeys[i]);
-	if (i < n)
-		atomicMax(reinterpret_cast<unsigned long long*>(out + 4),
-		          (unsigned long long)cbase[i] + (unsigned long long)(cu[i] + 1) * (unsigned long long)(cv[i] + 1));
+	// 64-bit maxima at one address are not merged by the compiler as the line
+	// above is: one per block (200,000 grids: the submission takes 344 us, 469
+	// with one per grid)
+	__shared__ unsigned long long blk;
+	if (threadIdx.x == 0) blk = 0;
+	__syncthreads();
+	unsigned long long last = 0;
+	if (i < n) last = (unsigned long long)cbase[i] + (unsigned long long)(cu[i] + 1) * (unsigned long long)(cv[i] + 1);
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) {
+		const unsigned long long other = __shfl_xor_sync(0xffffffffu, last, o);
+		last = other > last ? other : last;
+	}
+	if ((threadIdx.x & 31) == 0) atomicMax(&blk, last);
+	__syncthreads();
+	if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned long long*>(out + 4), blk);
 }
 }  // namespace
 
