@@ -1393,6 +1393,9 @@ sample_near_kernel(FrameParams fp, const __grid_constant__ GridsDev g, SamplerDe
 		if (!PERSIST) break;
 		continue;
 	}
+	// every warp has counted sm.bad before one sets more bits below: the count
+	// decides for the whole block which of its barriers come next
+	__syncthreads();
 
 	// ---- the samples, pixel-major: undecided ones are noted; the rest are
 	// resolved, or handed to resolve_opaque_kernel ----
