@@ -325,6 +325,10 @@ struct aqh_ctx {
 	cudaStream_t cstream = nullptr;
 	cudaEvent_t ev_before_up = nullptr, ev_cioi = nullptr;
 	cudaEvent_t ev_tables = nullptr;  // the grid tables' page-locked block has gone up
+	// everything the main stream reads from host memory for the last frame has
+	// been read (colours of packed grids: ev_cioi)
+	cudaEvent_t ev_inputs = nullptr;
+	bool staged_in_use = false;  // the last frame may still be reading hP, hCi and hOi
 	PinnedBuf h_tables;
 	DevBuf d_tables;
 	bool cioi_pending = false;
@@ -504,6 +508,7 @@ aqh_status aqh_create(const aqh_device_opts* opts, aqh_ctx** out) {
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_before_up, cudaEventDisableTiming);
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_cioi, cudaEventDisableTiming);
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_tables, cudaEventDisableTiming);
+	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_inputs, cudaEventDisableTiming);
 	if (e != cudaSuccess) {
 		delete ctx;
 		return e == cudaErrorMemoryAllocation ? AQH_ENOMEM : AQH_EDEVICE;
@@ -523,6 +528,7 @@ void aqh_destroy(aqh_ctx* ctx) {
 	if (ctx->ev_before_up) cudaEventDestroy(ctx->ev_before_up);
 	if (ctx->ev_cioi) cudaEventDestroy(ctx->ev_cioi);
 	if (ctx->ev_tables) cudaEventDestroy(ctx->ev_tables);
+	if (ctx->ev_inputs) cudaEventDestroy(ctx->ev_inputs);
 	if (ctx->cstream) cudaStreamDestroy(ctx->cstream);
 	for (auto& ge : ctx->graphs) cudaGraphExecDestroy(ge.exec);
 	if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
@@ -678,6 +684,10 @@ aqh_status aqh_submit_grid(aqh_ctx* ctx, const aqh_grid* gr) {
 	const int64_t nv = (int64_t)(gr->cu + 1) * (gr->cv + 1);
 	const int64_t nmp = (int64_t)gr->cu * gr->cv;
 	if (ctx->h_mps + nmp > INT32_MAX) return ctx->fail(AQH_ELIMIT, "more than 2^31 micropolygons in one frame");
+	if (ctx->staged_in_use) {
+		AQH_TRY(cudaEventSynchronize(ctx->ev_inputs), "stage grid");
+		ctx->staged_in_use = false;
+	}
 	ctx->h_cu.push_back(gr->cu);
 	ctx->h_cv.push_back(gr->cv);
 	ctx->h_nkeys.push_back(gr->nkeys);
@@ -1083,6 +1093,14 @@ static aqh_status upload_host_grids(aqh_ctx* ctx) {
 }
 
 
+// Waits until the host memory of the frame just queued has been read.
+static aqh_status inputs_read(aqh_ctx* ctx) {
+	AQH_TRY(cudaEventSynchronize(ctx->ev_inputs), "uploads");
+	if (ctx->host_packed) AQH_TRY(cudaEventSynchronize(ctx->ev_cioi), "uploads");
+	ctx->staged_in_use = false;
+	return AQH_OK;
+}
+
 static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	FrameParams& fp = ctx->fp;
 	cudaStream_t s = ctx->stream;
@@ -1091,6 +1109,7 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 		st = upload_packed_grids(ctx);
 		if (st != AQH_OK) return st;
 	} else if (!ctx->dev_grids) {
+		ctx->staged_in_use = true;
 		st = upload_host_grids(ctx);
 		if (st != AQH_OK) return st;
 	}
@@ -1653,7 +1672,11 @@ aqh_status aqh_render(aqh_ctx* ctx, int sync) {
 	RenderPlan P;
 	std::memset(static_cast<void*>(&P), 0, sizeof P);  // graphs are found by its bytes, padding included
 	aqh_status st = plan_render(ctx, P);
-	if (st != AQH_OK) return st;
+	AQH_TRY(cudaEventRecord(ctx->ev_inputs, ctx->stream), "uploads");
+	if (st != AQH_OK) {
+		inputs_read(ctx);
+		return st;
+	}
 	ctx->stats.micropolygons = P.nmps;
 	ctx->stats.samples = (int64_t)P.nsamp;
 	ctx->stats.grids = P.g.ngrids;
@@ -1661,7 +1684,11 @@ aqh_status aqh_render(aqh_ctx* ctx, int sync) {
 	// so do frames with trim curves (their micropolygon marks are per frame)
 	if (ctx->mode == AQH_MODE_BATCHED && P.g.csg.nnodes == 0 && P.g.trim.nsets == 0 && !ctx->cull_on)
 		return render_batched(ctx, P, sync != 0);
-	return render_plain(ctx, P, sync != 0 || P.g.csg.nnodes > 0);
+	st = render_plain(ctx, P, sync != 0 || P.g.csg.nnodes > 0);
+	// the caller may reuse its arrays once the plain form returns; by now the
+	// whole frame is queued, so the wait leaves the device no gap
+	const aqh_status in = inputs_read(ctx);
+	return st != AQH_OK ? st : in;
 }
 
 aqh_status aqh_synchronize(aqh_ctx* ctx) {

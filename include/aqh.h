@@ -208,8 +208,11 @@ aqh_status aqh_submit_grids_device(aqh_ctx* ctx, int ngrids,
                                    const uint8_t* d_culled, int64_t total_micropolygons);
 /* Append many grids from packed HOST arrays (same layout as
  * aqh_submit_grids_device).  Nothing is copied until aqh_render, which
- * uploads them in one transfer per array; the arrays must stay valid until
- * then.  Page-locked memory (aqh_host_alloc) transfers fastest. */
+ * uploads them in one transfer per array; the arrays must stay valid until it
+ * has read them.  The plain form (aqh_set_mode) has when it returns.  The
+ * batched form with sync = 0 does not wait for transfers: page-locked arrays
+ * belong to the frame until aqh_synchronize or a read of its results.
+ * Page-locked memory (aqh_host_alloc) transfers fastest. */
 aqh_status aqh_submit_grids_host(aqh_ctx* ctx, int ngrids,
                                  const int32_t* cu, const int32_t* cv, const int32_t* nkeys,
                                  const int32_t* flags, const int64_t* pbase, const int64_t* cbase,
@@ -244,8 +247,11 @@ aqh_status aqh_set_stream(aqh_ctx* ctx, void* stream);
  * (bucketprocessor.cpp:95-359) done on the device.  Asynchronous on the
  * context's stream unless `sync` is nonzero. */
 aqh_status aqh_render(aqh_ctx* ctx, int sync);
-/* Execution form of aqh_render.  PLAIN: one launch per stage, the host reads
- * binning's list size and the fragment count back between stages.  BATCHED:
+/* Execution form of aqh_render.  PLAIN: one launch per stage; between stages
+ * the host reads back the fragment count of transparent frames, and binning's
+ * list size where grids times super-tiles exceed 2^21 (smaller frames reserve
+ * room for that many list entries); it returns once the frame's host arrays
+ * have been read.  BATCHED:
  * a persistent sampling kernel pulls tiles from a device work queue, nothing
  * synchronizes with the host inside a frame, and the frame's whole
  * bin -> sample -> filter -> quantize sequence is one CUDA graph, captured on
@@ -416,7 +422,8 @@ aqh_status aqh_set_trim(aqh_ctx* ctx, const int32_t* grid_set, int ngrids, const
 #define AQH_MAX_AOV 16
 aqh_status aqh_set_aov_count(aqh_ctx* ctx, int n);
 /* Values for packed grids, float[vertices][n] indexed like Ci (cbase):
- * host arrays (kept by the caller until aqh_render returns) or device. */
+ * host arrays (kept by the caller as long as those of aqh_submit_grids_host)
+ * or device. */
 aqh_status aqh_submit_aov_host(aqh_ctx* ctx, const float* aov, size_t nvertices);
 aqh_status aqh_submit_aov_device(aqh_ctx* ctx, const float* d_aov);
 /* The filtered output variables of the crop window: float[h][w][n].  In
