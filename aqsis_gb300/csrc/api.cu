@@ -427,9 +427,12 @@ struct aqh_ctx {
 	bool graph_valid = true;  // false: buffers moved, drop every cached graph
 	int64_t graphs_built = 0, overflow_rerenders = 0;
 	bool pending_check = false;
-	// plain frames that did not wait for binning: where their list entries' number is
-	bool pairs_pending = false;
+	// plain frames that did not wait for binning: where their list entries'
+	// number is, on the device or (frames not waited for) in h_pairs after ev_pairs
+	bool pairs_pending = false, pairs_on_host = false;
 	const int32_t* pairs_at = nullptr;
+	PinnedBuf h_pairs;
+	cudaEvent_t ev_pairs = nullptr;
 	aqh::RenderPlan pending_plan{};
 	// sampler
 	DevBuf s_pos, s_time, s_dof, s_shuffle, s_lod, s_ipos, s_idof, s_itime, s_ishuf, s_ilod, s_dither;
@@ -509,6 +512,7 @@ aqh_status aqh_create(const aqh_device_opts* opts, aqh_ctx** out) {
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_cioi, cudaEventDisableTiming);
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_tables, cudaEventDisableTiming);
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_inputs, cudaEventDisableTiming);
+	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_pairs, cudaEventDisableTiming);
 	if (e != cudaSuccess) {
 		delete ctx;
 		return e == cudaErrorMemoryAllocation ? AQH_ENOMEM : AQH_EDEVICE;
@@ -529,6 +533,7 @@ void aqh_destroy(aqh_ctx* ctx) {
 	if (ctx->ev_cioi) cudaEventDestroy(ctx->ev_cioi);
 	if (ctx->ev_tables) cudaEventDestroy(ctx->ev_tables);
 	if (ctx->ev_inputs) cudaEventDestroy(ctx->ev_inputs);
+	if (ctx->ev_pairs) cudaEventDestroy(ctx->ev_pairs);
 	if (ctx->cstream) cudaStreamDestroy(ctx->cstream);
 	for (auto& ge : ctx->graphs) cudaGraphExecDestroy(ge.exec);
 	if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
@@ -1514,6 +1519,10 @@ static aqh_status render_plain(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 		if (wait) {
 			AQH_TRY(cudaMemcpyAsync(&total, ctx->pairs_at, 4, cudaMemcpyDeviceToHost, s), "readback");
 			AQH_TRY(cudaStreamSynchronize(s), "bin");
+		} else if (!sync) {
+			AQH_TRY(ctx->h_pairs.reserve(sizeof total), "readback");
+			AQH_TRY(cudaMemcpyAsync(ctx->h_pairs.p, ctx->pairs_at, 4, cudaMemcpyDeviceToHost, s), "readback");
+			AQH_TRY(cudaEventRecord(ctx->ev_pairs, s), "readback");
 		}
 	}
 	AQH_TRY(ctx->d_stlist.ensure(sizeof(int32_t) * std::max<int64_t>(wait ? total : most, 1)), "alloc tile lists");
@@ -1590,6 +1599,7 @@ static aqh_status render_plain(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 	cudaEventRecord(ctx->ev[3], s);
 	ctx->stats.tile_grid_pairs = total;
 	ctx->pairs_pending = !wait && P.g.ngrids > 0;  // aqh_get_stats reads them
+	ctx->pairs_on_host = !sync;
 	if (sync) {
 		AQH_TRY(cudaStreamSynchronize(s), "render");
 		read_stage_times(ctx);
@@ -2168,8 +2178,14 @@ aqh_status aqh_get_stats(aqh_ctx* ctx, aqh_frame_stats* st) {
 	if (ctx->pairs_pending) {
 		cudaSetDevice(ctx->device);
 		int32_t total = 0;
-		AQH_TRY(cudaMemcpyAsync(&total, ctx->pairs_at, 4, cudaMemcpyDeviceToHost, ctx->stream), "readback");
-		AQH_TRY(cudaStreamSynchronize(ctx->stream), "readback");
+		if (ctx->pairs_on_host) {
+			// waits for binning, not for the frame
+			AQH_TRY(cudaEventSynchronize(ctx->ev_pairs), "readback");
+			total = *static_cast<const int32_t*>(ctx->h_pairs.p);
+		} else {
+			AQH_TRY(cudaMemcpyAsync(&total, ctx->pairs_at, 4, cudaMemcpyDeviceToHost, ctx->stream), "readback");
+			AQH_TRY(cudaStreamSynchronize(ctx->stream), "readback");
+		}
 		ctx->stats.tile_grid_pairs = total;
 		ctx->pairs_pending = false;
 	}

@@ -4,6 +4,7 @@ some milliseconds goes first, so the next frame's uploads are still queued when
 its aqh_render returns.  (Its sample tables are below 64 KB: larger ones in
 pageable memory make aqh_set_samples wait for the device.)"""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -148,6 +149,27 @@ def test_next_frame_of_single_grids_leaves_the_last_one_alone(aqh_lib, batched):
         h.submit_scene_grids(b.grids)
         h.synchronize()
         assert _same(h.read_channels(), want[0])
+        del keep
+    finally:
+        h.close()
+
+
+def test_stats_do_not_wait_for_the_frame(aqh_lib):
+    """The list entries are known after binning, long before the frame is done."""
+    h = aqh_lib.Hider(0)
+    try:
+        sc, keep = _busy(h)
+        h.synchronize()
+        want = h.stats()["tile_grid_pairs"]
+        for _ in range(5):
+            h.render(sync=False)
+            t0 = time.perf_counter()
+            got = h.stats()["tile_grid_pairs"]
+            t1 = time.perf_counter()
+            h.synchronize()
+            t2 = time.perf_counter()
+            assert got == want
+        assert t1 - t0 < t2 - t1, (t1 - t0, t2 - t1)
         del keep
     finally:
         h.close()
