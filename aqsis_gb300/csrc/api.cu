@@ -1185,8 +1185,9 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	bb.st_offset = ctx->d_stoffset.as<int32_t>();
 	if (P.mbdof && P.nmps > 0) {
 		// each micropolygon's staging bound, computed once instead of in every tile it may reach
-		// (followed by its path where some grid has two keys and none has more)
-		bb.mp_stride = fp.max_keys == 2 ? 2 : 1;
+		// (followed by its path where some grid has two keys and none has more,
+		// and the path bounds the samples that can hit: offsets_bounded)
+		bb.mp_stride = fp.max_keys == 2 && offsets_bounded(fp, ctx->smp) ? 2 : 1;
 		AQH_TRY(ctx->d_mpb.ensure(sizeof(int4) * (size_t)P.nmps * bb.mp_stride), "alloc staging bounds");
 		bb.mp_bounds = ctx->d_mpb.as<int4>();
 	}

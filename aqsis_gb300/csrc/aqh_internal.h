@@ -128,6 +128,14 @@ struct SamplerDev {
 	int pos_unit;  // every position offset is a number in [0, 1] (checked on the host)
 };
 
+// Every sample lies in its pixel and every lens offset in the unit disc, so a
+// hit lies where the micropolygon is at the sample's time, give or take its
+// circle of confusion.  Frames of other samples keep every tile and time slice
+// whose bounds the reference visits: it tests a sample wherever its pixel is.
+__host__ __device__ inline bool offsets_bounded(const FrameParams& fp, const SamplerDev& smp) {
+	return smp.pos_unit && (!fp.use_dof || smp.dof_unit);
+}
+
 // Per-sample resolved store (after Combine): R G B depth / OR OG OB flags.
 // Sample store layout: sample-region pixels in blocks of 32 consecutive ones,
 // each block holding its samples sample-index-major ([block][sample][32]).
