@@ -657,7 +657,10 @@ sample_static_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 // alike the hit is a fragment or not; where they differ (an occluding
 // candidate of the same round covers the sample) the lane takes z from the
 // occluding candidates before the hit's own, found in the pixel's candidate
-// mask.  Flagged samples replay both kinds in order.  Fragments go to the
+// mask: the least of prev and their hits' depths.  Those with b above prev are
+// left out (the reference skips them, and their hits can round to below prev);
+// of the others an unflagged sample has no hit below b, so one that early-z
+// skips lies above z and does not change the least.  Flagged samples replay both kinds in order.  Fragments go to the
 // pool in any order (Combine sorts them), and Combine runs as its own kernel.
 // The ordered kernel these frames took before (a warp walks the union of 32
 // samples' candidates one after another, then combines with little L1 left)
@@ -953,7 +956,8 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 				if (zp <= D) return;
 				app = !(r.bminz > zk) && !(zk <= D);
 				if (!app) {
-					// z after the occluding candidates before this one
+					// z after the occluding candidates before this one (those
+					// behind prev fail early-z there too, wherever they are hit)
 					float z = zp;
 					for (int wd = 0; wd <= (lo >> 5); ++wd) {
 						uint32_t mb = sm.mask[pl][wd];
@@ -962,7 +966,8 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 							const int c = wd * 32 + __ffs(mb) - 1;
 							mb &= mb - 1u;
 							float Dc, uc, vc;
-							if (static_hit(fp, g, smp, bb, sm.rec[c], px, py, si, x, y, Dc, uc, vc)) z = fminf(z, Dc);
+							if (!(sm.rec[c].bminz > zp) && static_hit(fp, g, smp, bb, sm.rec[c], px, py, si, x, y, Dc, uc, vc))
+								z = fminf(z, Dc);
 						}
 					}
 					app = !(r.bminz > z) && !(z <= D);

@@ -936,7 +936,8 @@ sample_mb_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Samp
 // move z, so it lies between the round's start (prev) and, of a sample no
 // occluding hit flagged, the round's end (key): where the two decide alike the
 // hit is a fragment or not, and where they differ the warp takes z from the
-// sample's occluding hits of the candidates before it.  Flagged samples
+// sample's occluding hits of the candidates before it whose b is not above prev
+// (as in the static sampler, where the reason stands).  Flagged samples
 // replay both kinds in order.  640x480, 16 samples, motion blur + depth of
 // field, half of one layer transparent: 16.6 ms on the ordered kernel (one
 // sample per lane, slices one after another, one CTA per SM), 4.7 ms here.
@@ -1655,7 +1656,8 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 						const int px = tpx0 + pl % fp.tile_w, py = tpy0 + pl / fp.tile_w;
 						const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
 						const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s_]);
-						float z = key_depth_m(sm.prev[s_]);
+						const float zp = key_depth_m(sm.prev[s_]);
+						float z = zp;
 						for (int c0 = 0; c0 < c_; c0 += 32) {
 							const int cc = c0 + lane;
 							float Dc, bz;
@@ -1663,7 +1665,8 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 							if (cc < c_ && (sm.rec[cc].bits & 2) &&
 							    mb_hits_call(fp, g, smp, bb, sm.rec[cc], slice_times, sm.dofb[sm.kinv[s_]], px, py, j,
 							            make_float2((float)px + o.x, (float)py + o.y), sm.stime[s_], d, INFINITY, Dc, uvc,
-							            bz) > 0)
+							            bz) > 0 &&
+							    !(bz > zp))
 								z = fminf(z, Dc);
 						}
 #pragma unroll
