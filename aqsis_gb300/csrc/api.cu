@@ -1450,7 +1450,7 @@ static aqh_status enqueue_frame(aqh_ctx* ctx, RenderPlan& P, bool batched, bool 
 		AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
 	}
 	if (P.pool.capacity > 0) {
-		AQH_TRY(cudaMemsetAsync(P.pool.count, 0, 8, s), "memset");
+		AQH_TRY(cudaMemsetAsync(P.pool.count, 0, 16, s), "memset");
 		AQH_TRY(cudaMemsetAsync(P.pool.overflow, 0, 4, s), "memset");
 	}
 	if (timing) mark(ctx->ev[1]);
@@ -1540,7 +1540,7 @@ static aqh_status render_plain(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 	if (P.g.ngrids <= 0) AQH_TRY(cudaMemsetAsync(P.bb.st_offset, 0, sizeof(int32_t) * ((size_t)P.nst * P.bb.nranges + 1), s), "memset");
 	for (int attempt = 0; attempt < 4; ++attempt) {
 		if (P.pool.capacity > 0) {
-			AQH_TRY(cudaMemsetAsync(P.pool.count, 0, 8, s), "memset");
+			AQH_TRY(cudaMemsetAsync(P.pool.count, 0, 16, s), "memset");
 			AQH_TRY(cudaMemsetAsync(P.pool.overflow, 0, 4, s), "memset");
 		}
 		if (P.g.csg.nnodes > 0) AQH_TRY(cudaMemsetAsync(P.g.csg.overflow, 0, 4, s), "memset");
@@ -1556,11 +1556,12 @@ static aqh_status render_plain(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 		AQH_TRY(cudaGetLastError(), "sample kernel launch");
 		if (P.pool.capacity == 0) break;
 		int32_t ovf = 0;
-		unsigned long long used = 0;
+		unsigned long long count[2] = {0, 0};  // slots handed out, and those of them left empty
 		AQH_TRY(cudaMemcpyAsync(&ovf, P.pool.overflow, 4, cudaMemcpyDeviceToHost, s), "readback");
-		AQH_TRY(cudaMemcpyAsync(&used, P.pool.count, 8, cudaMemcpyDeviceToHost, s), "readback");
+		AQH_TRY(cudaMemcpyAsync(count, P.pool.count, sizeof count, cudaMemcpyDeviceToHost, s), "readback");
 		AQH_TRY(cudaStreamSynchronize(s), "sample");
-		ctx->stats.fragments = (int64_t)used;
+		const unsigned long long used = count[0];
+		ctx->stats.fragments = (int64_t)(used - count[1]);
 		if (!ovf) break;
 		// grow the fragment pool to what this frame needed and sample again
 		if (used > (unsigned long long)INT32_MAX)
@@ -1715,10 +1716,10 @@ aqh_status aqh_synchronize(aqh_ctx* ctx) {
 			AQH_TRY(cudaMemcpy(&total, P.bb.st_offset + (size_t)P.nst * P.bb.nranges, 4, cudaMemcpyDeviceToHost), "readback");
 		int32_t ovf = 0;
 		if (P.pool.capacity > 0) {
-			unsigned long long used = 0;
+			unsigned long long count[2] = {0, 0};
 			AQH_TRY(cudaMemcpy(&ovf, P.pool.overflow, 4, cudaMemcpyDeviceToHost), "readback");
-			AQH_TRY(cudaMemcpy(&used, P.pool.count, 8, cudaMemcpyDeviceToHost), "readback");
-			ctx->stats.fragments = (int64_t)used;
+			AQH_TRY(cudaMemcpy(count, P.pool.count, sizeof count, cudaMemcpyDeviceToHost), "readback");
+			ctx->stats.fragments = (int64_t)(count[0] - count[1]);
 		}
 		ctx->stats.tile_grid_pairs = total;
 		read_stage_times(ctx);

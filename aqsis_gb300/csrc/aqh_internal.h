@@ -177,7 +177,7 @@ struct SampleStore {
 struct FragPool {
 	float4* frag;
 	int32_t* next;
-	unsigned long long* count;
+	unsigned long long* count;  // slots handed out; [1]: of them left empty (holes of the samplers' runs)
 	int64_t capacity;
 	int32_t* overflow;
 	int32_t* occluders;  // nonzero when some micropolygon may be occluding (opaque or matte alpha)

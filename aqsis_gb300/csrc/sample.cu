@@ -668,7 +668,6 @@ sample_static_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 // transparent layers, against 1.97 ms here and 0.95 ms for Combine.
 constexpr int kSlotsO = 192;
 constexpr int kSlotsMix = 160;  // fewer: the candidate masks share the same shared memory
-constexpr int kMixRun = 64;     // pool slots a warp reserves at a time (at least 32)
 
 // Division of k < 2^16 by 1 <= d < 2^16 with a multiply: m = ceil(2^32 / d)
 // makes floor(k * m / 2^32) exact (the error k * (m - 2^32/d) / 2^32 < 2^-16 <
@@ -750,20 +749,15 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 	// MIXED: append the fragments of the lanes with `app` (one per lane, sample
 	// index `at` in pool.heads) from pool slots this warp reserved (a run's rest
 	// is used before the next run is reserved).
-	unsigned long long rnext = 0;
-	int rleft = 0;
+	FragRun run;
+	const int run_len = frag_run(fp.tile_w * fp.tile_h * fp.spp);
 	auto append = [&](bool app, long long at, float D, int id, float u, float v) {
 		const unsigned bal = __ballot_sync(0xffffffffu, app);
 		const int nh = __popc(bal), lane = threadIdx.x & 31;
 		if (nh == 0) return;
-		unsigned long long base = 0;
-		if (nh > rleft) {
-			if (lane == 0) base = atomicAdd(pool.count, (unsigned long long)kMixRun);
-			base = __shfl_sync(0xffffffffu, base, 0);
-		}
+		const unsigned long long base = run.reserve(pool, nh, run_len, lane);
 		if (app) {
-			const int rank = __popc(bal & ((1u << lane) - 1u));
-			const long long idx = (long long)(rank < rleft ? rnext + rank : base + (rank - rleft));
+			const long long idx = run.slot(__popc(bal & ((1u << lane) - 1u)), base);
 			if (idx < pool.capacity) {
 				pool.frag[idx] = make_float4(D, __int_as_float(id), u, v);
 				pool.next[idx] = atomicExch(pool.heads + at, (int)idx);
@@ -771,13 +765,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 				atomicOr(pool.overflow, 1);
 			}
 		}
-		if (nh > rleft) {
-			rnext = base + (nh - rleft);
-			rleft = kMixRun - (nh - rleft);
-		} else {
-			rnext += nh;
-			rleft -= nh;
-		}
+		run.used(nh, run_len, base);
 	};
 	for (int job = 0;; ++job) {
 	int tile;
@@ -1123,6 +1111,7 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 	}
 	}  // tile loop
+	if (MIXED) count_holes(pool, run.left);
 }
 
 // ---- opaque frames sampled near to far ----

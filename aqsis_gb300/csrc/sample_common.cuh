@@ -23,6 +23,51 @@ __device__ __forceinline__ unsigned long long near_key(float z, int w, bool anom
 }
 __device__ __forceinline__ int near_winner(unsigned long long k) { return (int)((uint32_t)k >> 1) - 1; }
 
+// Pool slots a warp of a tile of `tsamp` samples reserves at a time: the rest
+// of its last run stays empty, at most 16 warps' in a tile, which is less than
+// one slot in eight of the two per sample the pool holds at first.
+__device__ __forceinline__ int frag_run(int tsamp) { return max(4, min(64, tsamp >> 6)); }
+
+// Slots for the `nh` fragments of a warp: [next, next + left) are the rest of
+// its run, `base` the start of the run reserved now (when nh > left).
+struct FragRun {
+	unsigned long long next = 0;
+	int left = 0;
+	// the slot of the fragment of rank `rank`
+	__device__ __forceinline__ long long slot(int rank, unsigned long long base) const {
+		return (long long)(rank < left ? next + rank : base + (rank - left));
+	}
+	// `lane` of the whole warp; returns the new run's start
+	__device__ __forceinline__ unsigned long long reserve(const FragPool& pool, int nh, int run, int lane) const {
+		unsigned long long base = 0;
+		if (nh > left) {
+			if (lane == 0) base = atomicAdd(pool.count, (unsigned long long)max(run, nh - left));
+			base = __shfl_sync(0xffffffffu, base, 0);
+		}
+		return base;
+	}
+	__device__ __forceinline__ void used(int nh, int run, unsigned long long base) {
+		if (nh > left) {
+			next = base + (nh - left);
+			left = max(run, nh - left) - (nh - left);
+		} else {
+			next += nh;
+			left -= nh;
+		}
+	}
+};
+
+// Adds the empty rests of a block's runs to pool.count[1].
+__device__ __forceinline__ void count_holes(const FragPool& pool, int left) {
+	__shared__ int holes;
+	__syncthreads();
+	if (threadIdx.x == 0) holes = 0;
+	__syncthreads();
+	if ((threadIdx.x & 31) == 0 && left > 0) atomicAdd(&holes, left);
+	__syncthreads();
+	if (threadIdx.x == 0 && holes > 0) atomicAdd(pool.count + 1, (unsigned long long)holes);
+}
+
 // The level-of-detail test of RenderMPG_Static / RenderMPG_MBOrDof
 // (bucketprocessor.cpp:1182-1190, 1404-1412, 1439-1447): a grid whose
 // LevelOfDetailBounds minimum is >= 0 (the attribute defaults to 0 1,

@@ -1125,7 +1125,6 @@ constexpr int kItemsQ = 192;     // kept (candidate, slice) items per pass (at m
 constexpr int kTileSampQ = 2048;
 constexpr int kTilePixQ = 256;
 constexpr int kBinsQ = 64;       // time bins of a pixel at most
-constexpr int kFragRunQ = 64;    // pool slots a warp reserves at a time (at least 32: one drain's hits)
 constexpr int kBinTabQ = kTileSampQ + kTilePixQ;  // (bins + 1) entries per pixel, over the tile
 
 // One kept (candidate, slice) item of a pass.  Its sample slots are the
@@ -1461,22 +1460,17 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 	const bool any_nan = sm.any_nan != 0;
 
 	// TRANSP: append fragments of the lanes with `app` (one per lane) to their
-	// samples' lists.  Pool slots come in runs of kFragRunQ a warp reserves with
-	// one atomic (a run's rest is used before the next is reserved).
-	unsigned long long rnext = 0;
-	int rleft = 0;
+	// samples' lists.  Pool slots come in runs a warp reserves with one atomic (a
+	// run's rest is used before the next is reserved).
+	FragRun run;
+	const int run_len = frag_run(tsamp);
 	auto append = [&](bool app, int s, float D, int id, float u, float v) {
 		const unsigned bal = __ballot_sync(0xffffffffu, app);
 		const int nh = __popc(bal);
 		if (nh == 0) return;
-		unsigned long long base = 0;
-		if (nh > rleft) {
-			if (lane == 0) base = atomicAdd(pool.count, (unsigned long long)kFragRunQ);
-			base = __shfl_sync(0xffffffffu, base, 0);
-		}
+		const unsigned long long base = run.reserve(pool, nh, run_len, lane);
 		if (app) {
-			const int rank = __popc(bal & ((1u << lane) - 1u));
-			const long long idx = (long long)(rank < rleft ? rnext + rank : base + (rank - rleft));
+			const long long idx = run.slot(__popc(bal & ((1u << lane) - 1u)), base);
 			if (idx < pool.capacity) {
 				pool.frag[idx] = make_float4(D, __int_as_float(id), u, v);
 				pool.next[idx] = atomicExch(&sm.fhead[s], (int)idx);
@@ -1484,13 +1478,7 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 				atomicOr(pool.overflow, 1);
 			}
 		}
-		if (nh > rleft) {
-			rnext = base + (nh - rleft);
-			rleft = kFragRunQ - (nh - rleft);
-		} else {
-			rnext += nh;
-			rleft -= nh;
-		}
+		run.used(nh, run_len, base);
 	};
 
 	const int lbeg = bb.st_offset[st_idx * bb.nranges];
@@ -1915,6 +1903,7 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 		if (st.wmask) st.wmask[store_index(pix, j, spp)] =
 		    window_word(fp, px, py, (float)px + o.x, (float)py + o.y, has);
 	}
+	if (TRANSP) count_holes(pool, run.left);
 }
 
 }  // namespace

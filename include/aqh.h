@@ -492,7 +492,8 @@ typedef struct {
 	int64_t samples;              /* samples in the sample region */
 	int64_t grids;
 	int64_t tile_grid_pairs;      /* grid references the tile lists hold */
-	int64_t fragments;            /* transparent fragments stored */
+	int64_t fragments;            /* transparent fragments stored (static frames without an opaque
+	                                 surface: the slots handed out for them, a few more) */
 	float ms_bin, ms_sample, ms_filter, ms_total;  /* device time per stage of the last render */
 	int64_t graphs_built;         /* batched mode: frame graphs captured by this context so far */
 	int64_t rerenders;            /* batched mode: frames rendered again on the plain path because
