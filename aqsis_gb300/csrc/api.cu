@@ -1421,7 +1421,6 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 }
 
 static const int kDefaultDisplay[4] = {0, 1, 2, 6};  // r, g, b, a
-constexpr int64_t kListBound = 1 << 21;  // list entries (8 MB) a plain frame reserves without asking for their number
 
 // The device work of one frame after binning's list capacity is known.
 // `batched`: persistent sampling kernel fed from a work queue; no host
@@ -1616,9 +1615,9 @@ constexpr size_t kMaxGraphs = 16;
 
 static aqh_status render_batched(aqh_ctx* ctx, RenderPlan& P, bool sync) {
 	cudaStream_t s = ctx->stream;
-	// list room for 16 super-tiles per grid: a frame that needs more is caught
-	// on the device and rendered again on the plain path
-	const int64_t want = std::max<int64_t>(ctx->st_list_cap, (int64_t)P.g.ngrids * 16 + 4096);
+	// a frame that needs more list entries is caught on the device and rendered
+	// again on the plain path
+	const int64_t want = std::max<int64_t>(ctx->st_list_cap, list_batched(P.g.ngrids));
 	AQH_TRY(ctx->d_stlist.ensure(sizeof(int32_t) * want), "alloc tile lists");
 	ctx->st_list_cap = ctx->d_stlist.cap / sizeof(int32_t);
 	P.bb.st_list = ctx->d_stlist.as<int32_t>();

@@ -213,6 +213,14 @@ struct BinBuffers {
 };
 constexpr int kIrrWords = 32;     // grids of more micropolygons than bits are not analysed
 constexpr int kRedoPerTile = 8;   // redo entries of a tile at most (more pixels: the whole tile)
+constexpr int64_t kListBound = 1 << 21;  // list entries (8 MB) a plain frame reserves without asking for their number
+// List entries a batched frame reserves at first: 16 super-tiles per grid.
+inline int64_t list_batched(int64_t ngrids) { return ngrids * 16 + 4096; }
+// The most entries either form reserves before it knows their number.
+inline int64_t list_room(int64_t ngrids, int nst) {
+	const int64_t most = ngrids * nst < kListBound ? ngrids * nst : kListBound;
+	return most > list_batched(ngrids) ? most : list_batched(ngrids);
+}
 
 // Camera-to-raster matrix of the frame in CqMatrix element order m[row*4 + col].
 struct CamMatrix {
