@@ -1258,11 +1258,12 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 			bb.grid_nirr = reinterpret_cast<int32_t*>(bb.grid_slack + G);
 			bb.irregular = ctx->d_irr.as<uint32_t>();
 		}
-		AQH_TRY(ctx->d_redo.ensure(sizeof(int32_t) * (3 + (size_t)kRedoPerTile * fp.ntx * fp.nty)), "alloc redo list");
+		AQH_TRY(ctx->d_redo.ensure(sizeof(int32_t) * (kRedoHead + (size_t)kRedoPerTile * fp.ntx * fp.nty)), "alloc redo list");
 		bb.redo_next = ctx->d_redo.as<int32_t>();
 		bb.nirr_total = bb.redo_next + 1;
 		bb.nirr_limit = (int32_t)(P.nmps / 8);
-		bb.redo = bb.redo_next + 2;
+		bb.near_tried = bb.redo_next + 2;
+		bb.redo = bb.redo_next + kRedoHead - 1;
 	}
 	if (pool.capacity == 0 && !P.mbdof && ctx->host_packed) {
 		// colours still on their way from the host: the sampler hands its

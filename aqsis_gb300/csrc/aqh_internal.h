@@ -210,8 +210,10 @@ struct BinBuffers {
 	int32_t* redo_next;    // entries of redo handed out
 	int32_t* nirr_total;   // irregular micropolygons of the frame; above nirr_limit all tiles go in
 	int32_t nirr_limit;    // grid order
+	int32_t* near_tried;   // tiles the near to far sampler has tried, and of them those it gave up
 };
 constexpr int kIrrWords = 32;     // grids of more micropolygons than bits are not analysed
+constexpr int kRedoHead = 5;      // counters in front of the redo entries
 constexpr int kRedoPerTile = 8;   // redo entries of a tile at most (more pixels: the whole tile)
 constexpr int64_t kListBound = 1 << 21;  // list entries (8 MB) a plain frame reserves without asking for their number
 // List entries a batched frame reserves at first: 16 super-tiles per grid.

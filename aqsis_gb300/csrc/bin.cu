@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(kDepthBuckets) depth_order_kernel(BinBuffers b
 }
 
 void launch_depth_order(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s) {
-	cudaMemsetAsync(b.redo_next, 0, 3 * sizeof(int32_t), s);  // with nirr_total and the redo count
+	cudaMemsetAsync(b.redo_next, 0, kRedoHead * sizeof(int32_t), s);  // every counter
 	if (g.ngrids == 0) return;
 	if (!b.grid_slack) {
 		// moving frames: the slacks come with the staging bounds

@@ -1149,7 +1149,16 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 // sample patterns twice the L1): every opaque static frame takes it.  Layers of
 // flat grids at random depths, where rounding makes 40% of the hits anomalous,
 // 15.0 -> 4.1; several layers in exactly one plane, which mostly go in order
-// after all, 19.0 -> 23.4.
+// after all, 19.0 -> 19.8.
+//
+// That last figure was 21.2 with every tile tried.  A tile given up costs a
+// tenth of its ordered time, so once 32 tiles and three quarters of those tried
+// were given up, the others go to the list untried, except one in 32, which
+// keeps the share current where the image changes.  Which tiles those are
+// depends on timing; the results do not.  Frames of up to 512 tiles, most of
+// which start before one is done, are not counted.
+constexpr int kCountedTiles = 512;
+
 struct RecZ : RecS {
 	float zcull;  // b - slack; -inf: never skipped
 	int pad;      // an odd number of words
@@ -1195,6 +1204,7 @@ sample_near_kernel(FrameParams fp, const __grid_constant__ GridsDev g, SamplerDe
 	SmemZ& sm = *reinterpret_cast<SmemZ*>(smem_raw);
 	__shared__ int next_tile;
 	const int ntiles = fp.ntx * fp.nty;
+	const bool counted = ntiles > kCountedTiles;
 	const FragPool nopool{};
 	for (int job = 0;; ++job) {
 	int tile;
@@ -1218,6 +1228,11 @@ sample_near_kernel(FrameParams fp, const __grid_constant__ GridsDev g, SamplerDe
 	const uint32_t mxs = div_magic(xs), mys = div_magic(ys);
 	const int tpix = tw * th;
 	const int tsamp = tpix * spp;
+	int given = 0, tried = 0;
+	if (t == 0 && counted) {
+		tried = *(volatile int32_t*)bb.near_tried;
+		given = *(volatile int32_t*)(bb.near_tried + 1);
+	}
 	const unsigned long long kinit = near_key(FLT_MAX, -1, false);
 
 	for (int i = t; i < tsamp; i += kThreadsS) {
@@ -1242,9 +1257,14 @@ sample_near_kernel(FrameParams fp, const __grid_constant__ GridsDev g, SamplerDe
 	if (t == 0) {
 		sm.qn = 0;
 		sm.qcum[0] = 0;
-		sm.whole = 0;
+		sm.whole = (tile & 31) != 0 && given >= 32 && given > tried - (tried >> 2);  // not worth trying
 	}
 	__syncthreads();
+	if (sm.whole) {
+		if (t == 0) bb.redo[1 + atomicAdd(bb.redo, 1)] = tile;
+		if (!PERSIST) break;
+		continue;
+	}
 
 	const int lbeg = bb.st_offset[st_idx * bb.nranges];
 	const int lend = (int)min((long long)bb.st_offset[(st_idx + 1) * bb.nranges], (long long)bb.list_capacity);
@@ -1383,6 +1403,10 @@ sample_near_kernel(FrameParams fp, const __grid_constant__ GridsDev g, SamplerDe
 		undecided = sm.whole ? kRedoPerTile + 1 : 0;
 		for (int i = 0; i < kTilePixMax / 32; ++i) undecided += __popc(sm.bad[i]);
 		if (exhausted || undecided > kRedoPerTile) break;
+	}
+	if (t == 0 && counted) {
+		atomicAdd(bb.near_tried, 1);
+		if (undecided > kRedoPerTile) atomicAdd(bb.near_tried + 1, 1);
 	}
 	if (undecided > kRedoPerTile) {
 		if (t == 0) bb.redo[1 + atomicAdd(bb.redo, 1)] = tile;

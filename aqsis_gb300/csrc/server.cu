@@ -80,7 +80,7 @@ extern "C" size_t aqh_job_footprint(const aqh_job* j) {
 	b += j->nP * 16 + j->nC * 32 + (size_t)j->ngrids * (5 * 4 + 3 * 8) + j->ntimes * 4;  // grids
 	b += (size_t)j->ngrids * (16 + 4) + 65536;                                          // bin
 	const size_t tiles = (size_t)fp.ntx * fp.nty, lists = (size_t)aqh::list_room(j->ngrids, fp.nstx * fp.nsty);
-	b += lists * 8 + (3 + aqh::kRedoPerTile * tiles) * 4;                                // grid lists, in both orders; redo list
+	b += lists * 8 + (aqh::kRedoHead + aqh::kRedoPerTile * tiles) * 4;                                // grid lists, in both orders; redo list
 	if (j->culled) b += (size_t)j->micropolygons;                                        // culled flags
 	int max_keys = 0;
 	for (int i = 0; i < j->ngrids; ++i) max_keys = std::max(max_keys, (int)j->nkeys[i]);
