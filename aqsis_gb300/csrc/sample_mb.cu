@@ -1282,7 +1282,12 @@ __device__ __forceinline__ int quot(int r, uint32_t m) { return m == 0u ? r : (i
 // As sample_near_kernel (sample.cu), whose argument covers (slice, sample)
 // tests as well: a hit is kept when some slice that holds it passes early-z, so
 // its b is the least min z of those slices, and a hit is anomalous when D is
-// below the min z of every one (the key prefers the slice that is not).  No
+// below the min z of every one (the key prefers the slice that is not).  A
+// sample whose time lies on a slice's end meets the micropolygon in the next one
+// too, at the same depth: that is no second hit (counted as one it left a tile
+// undecided in most frames, which a redone tile takes twice as long in a small
+// one: 320x240, 16 samples, motion blur, 1.5 layers 744 us with it, 480 without).
+// No
 // hit of a micropolygon is nearer than its staging bound's least depth
 // (mb_hit_depth).  For an anomalous hit b is bounded by the micropolygon's
 // largest corner depth over all keys; a slice beyond the keys, whose bound is
@@ -1622,8 +1627,10 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 							} else {
 								const unsigned long long mine = near_key(D, r.id, D < b);
 								const unsigned long long was = atomicMin(&sm.key[s], mine);
-								// of the two the farther depth is another hit's
-								atomicMin(&sm.z2[s], max((uint32_t)(was >> 32), (uint32_t)(mine >> 32)));
+								// of the two the farther depth is another hit's, unless both
+								// are this micropolygon's, in two slices
+								if (((uint32_t)was ^ (uint32_t)mine) > 1u)
+									atomicMin(&sm.z2[s], max((uint32_t)(was >> 32), (uint32_t)(mine >> 32)));
 								if (mine < was) atomicOr(&sm.dirty[pl >> 5], 1u << (pl & 31));
 							}
 						} else if (!(D >= wz[lane]) || D == 0.0f) {
