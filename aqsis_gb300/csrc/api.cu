@@ -1462,7 +1462,7 @@ static aqh_status enqueue_frame(aqh_ctx* ctx, RenderPlan& P, bool batched, bool 
 		AQH_TRY(cudaStreamWaitEvent(s, ctx->ev_cioi, wflags), "wait for colours");
 		launch_sample_mb(fp, P.g, ctx->smp, P.bb, P.store, P.pool, ctx->d_dofb.as<float4>(), ctx->d_slices.as<float>(), s);
 	} else if (batched) {
-		AQH_TRY(cudaMemsetAsync(ctx->d_queue.p, 0, 4, s), "memset");
+		AQH_TRY(cudaMemsetAsync(ctx->d_queue.p, 0, 8, s), "memset");  // a counter for each of two samplers
 		launch_sample_tiles_q(fp, P.g, ctx->smp, P.bb, P.store, P.pool, ctx->d_queue.as<int>(), nullptr, P.nctas, s,
 		                      ctx->ev_cioi, wflags);
 	} else {
@@ -1684,7 +1684,12 @@ aqh_status aqh_render(aqh_ctx* ctx, int sync) {
 	RenderPlan P;
 	std::memset(static_cast<void*>(&P), 0, sizeof P);  // graphs are found by its bytes, padding included
 	aqh_status st = plan_render(ctx, P);
-	AQH_TRY(cudaEventRecord(ctx->ev_inputs, ctx->stream), "uploads");
+	// CSG frames take the plain path, which reads the resolve's overflow flag;
+	// so do frames with trim curves (their micropolygon marks are per frame)
+	const bool batched = ctx->mode == AQH_MODE_BATCHED && P.g.csg.nnodes == 0 && P.g.trim.nsets == 0 && !ctx->cull_on;
+	const bool whole = sync != 0 || (!batched && P.g.csg.nnodes > 0);  // wait for the whole frame
+	if (st != AQH_OK || (!whole && (!batched || ctx->staged_in_use)))
+		AQH_TRY(cudaEventRecord(ctx->ev_inputs, ctx->stream), "uploads");
 	if (st != AQH_OK) {
 		inputs_read(ctx);
 		return st;
@@ -1692,11 +1697,12 @@ aqh_status aqh_render(aqh_ctx* ctx, int sync) {
 	ctx->stats.micropolygons = P.nmps;
 	ctx->stats.samples = (int64_t)P.nsamp;
 	ctx->stats.grids = P.g.ngrids;
-	// CSG frames take the plain path, which reads the resolve's overflow flag;
-	// so do frames with trim curves (their micropolygon marks are per frame)
-	if (ctx->mode == AQH_MODE_BATCHED && P.g.csg.nnodes == 0 && P.g.trim.nsets == 0 && !ctx->cull_on)
-		return render_batched(ctx, P, sync != 0);
-	st = render_plain(ctx, P, sync != 0 || P.g.csg.nnodes > 0);
+	st = batched ? render_batched(ctx, P, whole) : render_plain(ctx, P, whole);
+	if (whole) {
+		if (st == AQH_OK) ctx->staged_in_use = false;
+		return st;
+	}
+	if (batched) return st;
 	// the caller may reuse its arrays once the plain form returns; by now the
 	// whole frame is queued, so the wait leaves the device no gap
 	const aqh_status in = inputs_read(ctx);

@@ -263,7 +263,7 @@ void launch_project_grids(const GridsDev& g, float4* P, int32_t* flags, const Ca
 void launch_st_count(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cudaStream_t s);
 void launch_scan_i32(const int32_t* in, int32_t* out, int n, int32_t* scratch, cudaStream_t s);
 void launch_st_write(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cudaStream_t s);
-// Fills st_sorted, grid_slack, grid_nirr and irregular, and empties redo.
+// Fills st_sorted, grid_slack, grid_nirr and irregular (launch_grid_rects has emptied redo).
 void launch_depth_order(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s);
 // `colours_ready`, when given, is an event the first kernel that reads Ci/Oi
 // waits for (on an opaque frame, the resolve after the sampler), with

@@ -83,7 +83,8 @@ __device__ __forceinline__ void grid_strips(const float4* P, int cu, int cv, int
 }
 
 __global__ void grid_rects_kernel(FrameParams fp, GridsDev g, int4* rect, float* minz, uint32_t* strips,
-                                  float4* tri) {
+                                  float4* tri, int32_t* redo_head) {
+	if (redo_head && blockIdx.x == 0 && threadIdx.x < kRedoHead) redo_head[threadIdx.x] = 0;
 	const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int lane = threadIdx.x & 31;
 	if (warp >= g.ngrids) return;
@@ -436,7 +437,8 @@ void launch_id_grid(const GridsDev& g, int64_t nmps, int32_t* table, cudaStream_
 void launch_grid_rects(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s) {
 	if (g.ngrids == 0) return;
 	const int wpb = kBlock / 32;
-	grid_rects_kernel<<<(g.ngrids + wpb - 1) / wpb, kBlock, 0, s>>>(fp, g, b.grid_rect, b.grid_minz, b.strips, b.tri);
+	grid_rects_kernel<<<(g.ngrids + wpb - 1) / wpb, kBlock, 0, s>>>(fp, g, b.grid_rect, b.grid_minz, b.strips, b.tri,
+	                                                                     b.redo_next);
 }
 
 void launch_st_count(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cudaStream_t s) {
@@ -625,7 +627,6 @@ __global__ void __launch_bounds__(kDepthBuckets) depth_order_kernel(BinBuffers b
 }
 
 void launch_depth_order(const FrameParams& fp, const GridsDev& g, const BinBuffers& b, cudaStream_t s) {
-	cudaMemsetAsync(b.redo_next, 0, kRedoHead * sizeof(int32_t), s);  // every counter
 	if (g.ngrids == 0) return;
 	if (!b.grid_slack) {
 		// moving frames: the slacks come with the staging bounds

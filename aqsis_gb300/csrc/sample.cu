@@ -1818,9 +1818,8 @@ void launch_sample_tiles_q(const FrameParams& fp, const GridsDev& g, const Sampl
 			if (n > 0) resolve_frag_kernel<<<(unsigned)nb, 256, 0, s>>>(fp, g, sm, st, pool);
 			if (mixed) {
 				if (queue) {
-					cudaMemsetAsync(queue, 0, sizeof(int), s);  // sample_frag_kernel may have drawn from it
-					sample_opaque_kernel<true, kSlotsMix, true><<<nctas, kThreadsS, sizeof(SmemMix), s>>>(fp, g, sm, b, st, pool,
-					                                                                                    queue, order);
+					sample_opaque_kernel<true, kSlotsMix, true><<<nctas, kThreadsS, sizeof(SmemMix), s>>>(
+					    fp, g, sm, b, st, pool, queue + 1, order);  // sample_frag_kernel may have drawn from the first
 				} else {
 					sample_opaque_kernel<false, kSlotsMix, true><<<ntiles, kThreadsS, sizeof(SmemMix), s>>>(
 					    fp, g, sm, b, st, pool, nullptr, nullptr);

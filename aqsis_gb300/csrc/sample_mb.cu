@@ -1287,8 +1287,7 @@ __device__ __forceinline__ int quot(int r, uint32_t m) { return m == 0u ? r : (i
 // too, at the same depth: that is no second hit (counted as one it left a tile
 // undecided in most frames, which a redone tile takes twice as long in a small
 // one: 320x240, 16 samples, motion blur, 1.5 layers 744 us with it, 480 without).
-// No
-// hit of a micropolygon is nearer than its staging bound's least depth
+// No hit of a micropolygon is nearer than its staging bound's least depth
 // (mb_hit_depth).  For an anomalous hit b is bounded by the micropolygon's
 // largest corner depth over all keys; a slice beyond the keys, whose bound is
 // extrapolated past that, leaves its tile undecided.  Undecided tiles, and
