@@ -1106,6 +1106,24 @@ static aqh_status inputs_read(aqh_ctx* ctx) {
 	return AQH_OK;
 }
 
+// Is the frame large enough for near to far sampling?  The order, the depth
+// bounds and the second sampler are four launches more (three in moving
+// frames), 10 to 15 us that the hidden micropolygons have to be worth.  Static
+// frames of at most 2^21 samples, ordered / near, device time (us): 320x240, 4
+// samples, unit quads 0.7 layers deep 126 / 129, 1.5 138 / 151, 4 214 / 201; 16
+// samples, 0.3 166 / 182, 0.7 218 / 211; 640x480, 1 sample, 1.5 248 / 263, 4 404
+// / 398.  Micropolygons times samples per pixel, per pixel, stand for the layers:
+// above 12 the order gains, above 24 in frames of few micropolygons (32x32, 16
+// samples, 1.3 layers 158 / 164, 3.5 207 / 184).  Larger frames take it
+// whatever their depth (640x480, 16 samples, 0.1 layers 291 / 306, 1.5 624 / 612:
+// quads wider than a pixel hide more than their number says).  Moving ones:
+// 96x64, 576 micropolygons 100 / 105, 1,792 116 / 116, 4,288 152 / 139.
+static bool near_pays(const RenderPlan& P, const FrameParams& fp) {
+	if (P.mbdof) return P.nmps >= 1024;
+	if (P.nsamp > (size_t)1 << 21) return true;
+	return (double)P.nmps * fp.spp >= (P.nmps < 16384 ? 24.0 : 12.0) * fp.sw * fp.sh;
+}
+
 static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	FrameParams& fp = ctx->fp;
 	cudaStream_t s = ctx->stream;
@@ -1248,7 +1266,7 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 			pool.heads = ctx->d_fheads.as<int32_t>();
 		}
 	}
-	if (pool.capacity == 0 && G > 0 && P.nmps > 0 && (!P.mbdof || ctx->smp.dof_unit)) {
+	if (pool.capacity == 0 && G > 0 && P.nmps > 0 && (!P.mbdof || ctx->smp.dof_unit) && near_pays(P, fp)) {
 		// sampled near to far (the depth bounds under depth of field take lens
 		// offsets inside the lens)
 		if (!P.mbdof) {

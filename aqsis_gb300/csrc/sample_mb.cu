@@ -1950,7 +1950,10 @@ void launch_sample_mb(const FrameParams& fp, const GridsDev& g, const SamplerDev
 		    fp, g, sm, b, st, pool, dof_bounds, slice_times);
 		sample_mbq_kernel<kMaxKeys, kSlotsQ, false, false, true><<<ntiles, kThreadsQ, sizeof(SmemQ), s>>>(
 		    fp, g, sm, b, st, pool, dof_bounds, slice_times);
-	} else
+	} else if (two)
+		sample_mbq_kernel<2, kSlotsQ2, false><<<ntiles, kThreadsQ, sizeof(SmemQ2), s>>>(fp, g, sm, b, st, pool, dof_bounds,
+		                                                                              slice_times);
+	else
 		sample_mbq_kernel<kMaxKeys, kSlotsQ, false><<<ntiles, kThreadsQ, sizeof(SmemQ), s>>>(fp, g, sm, b, st, pool,
 		                                                                                   dof_bounds, slice_times);
 }
@@ -1961,6 +1964,8 @@ void configure_sample_mb_kernels() {
 	if (!first_use_on_device(mu, configured)) return;
 	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemQ));
+	cudaFuncSetAttribute(sample_mbq_kernel<2, kSlotsQ2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     (int)sizeof(SmemQ2));
 	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)sizeof(SmemQN));
 	cudaFuncSetAttribute(sample_mbq_kernel<kMaxKeys, kSlotsQ, false, false, true>,

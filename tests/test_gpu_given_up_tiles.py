@@ -11,7 +11,7 @@ from tests.test_gpu_parity import compare
 pytestmark = pytest.mark.gpu
 
 
-def _scene(seed, flat, w=640, h=420, xs=2, layers=2.0):
+def _scene(seed, flat, w=640, h=420, xs=2, layers=4.0):
     """`flat`: which grids lie in one plane, by the position of their first vertex."""
     rng = np.random.default_rng(seed)
     fr = S.Frame(width=w, height=h, xsamples=xs, ysamples=xs, q_dither=0.0)
@@ -27,7 +27,7 @@ def _scene(seed, flat, w=640, h=420, xs=2, layers=2.0):
 
 CASES = {
     "all": (lambda x, y: x < 9.0, 2), "top": (lambda x, y: y < 0.7, 2), "bottom": (lambda x, y: y > 0.4, 2),
-    "stripes": (lambda x, y: (x * 5.0) % 1.0 < 0.8, 2), "none": (lambda x, y: x > 9.0, 2), "all_1x1": (lambda x, y: x < 9.0, 1),
+    "stripes": (lambda x, y: (x * 5.0) % 1.0 < 0.8, 2), "none": (lambda x, y: x > 9.0, 2), "all_3x3": (lambda x, y: x < 9.0, 3),
 }
 
 

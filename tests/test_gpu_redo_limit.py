@@ -37,7 +37,7 @@ def _scene(seed, xs, tiles=8):
 
 
 @pytest.mark.parametrize("batched", [False, True], ids=["plain", "batched"])
-@pytest.mark.parametrize("seed,xs", [(0, 2), (1, 4), (2, 4), (3, 4), (4, 1)])
+@pytest.mark.parametrize("seed,xs", [(0, 5), (1, 4), (2, 4), (3, 4), (4, 8)])
 def test_tiles_at_the_limit_match_oracle(aqh_lib, oracle, seed, xs, batched):
     sc = _scene(seed, xs)
     ref = oracle.render(sc)
