@@ -654,17 +654,19 @@ sample_static_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 // hits move: z lies between the round's start (prev) and, of a sample that no
 // occluding hit flagged, the round's end (key).  Where the two bounds decide
 // alike the hit is a fragment or not; where they differ (an occluding
-// candidate of the same round covers the sample) the lane takes z from the
-// occluding candidates before the hit's own, found in the pixel's candidate
-// mask: the least of prev and their hits' depths.  Those with b above prev are
-// left out (the reference skips them, and their hits can round to below prev);
-// of the others an unflagged sample has no hit below b, so one that early-z
-// skips lies above z and does not change the least.  Flagged samples replay both kinds in order.  Fragments go to the
-// pool in any order (Combine sorts them), and Combine runs as its own kernel.
-// The ordered kernel these frames took before (a warp walks the union of 32
-// samples' candidates one after another, then combines with little L1 left)
-// took 4.56 ms of a 1280x720 frame of 16 samples, 2.5 opaque and 0.8
-// transparent layers, against 1.97 ms here and 0.95 ms for Combine.
+// candidate of the same round covers the sample) it is none if the nearest
+// occluder comes before it (ids ascend in insertion order, and then z is at
+// most key's depth).  Else the lane takes z from the occluding candidates
+// before the hit's own, found in the pixel's candidate mask: the least of prev
+// and their hits' depths.  Those with b above prev are left out (the reference
+// skips them, and their hits can round to below prev); of the others an
+// unflagged sample has no hit below b, so one that early-z skips lies above z
+// and does not change the least.  Flagged samples replay both kinds in order.
+// Fragments go to the pool in any order (Combine sorts them), and Combine runs
+// as its own kernel. The ordered kernel these frames took before (a warp walks
+// the union of 32 samples' candidates one after another, then combines with
+// little L1 left) took 4.56 ms of a 1280x720 frame of 16 samples, 2.5 opaque
+// and 0.8 transparent layers, against 1.97 ms here and 0.95 ms for Combine.
 constexpr int kSlotsO = 192;
 constexpr int kSlotsMix = 160;  // fewer: the candidate masks share the same shared memory
 
@@ -941,10 +943,11 @@ sample_opaque_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, 
 			D = bilerp1(r.z[0], r.z[1], r.z[2], r.z[3], u, v);
 			if (!rec_keeps(g, bb, r.bits, r.id, x, y, u, v)) return;
 			if (MIXED && ph == 1) {
-				const float zp = key_depth(sm.prev[s]), zk = key_depth(sm.key[s]);
+				const unsigned long long kk = sm.key[s];
+				const float zp = key_depth(sm.prev[s]), zk = key_depth(kk);
 				if (zp <= D) return;
 				app = !(r.bminz > zk) && !(zk <= D);
-				if (!app) {
+				if (!app && key_winner(kk) > r.id) {
 					// z after the occluding candidates before this one (those
 					// behind prev fail early-z there too, wherever they are hit)
 					float z = zp;

@@ -935,12 +935,18 @@ sample_mb_kernel(FrameParams fp, GridsDev g, SamplerDev smp, BinBuffers bb, Samp
 // min z and z the occlZ at its place in insertion order.  Only occluding hits
 // move z, so it lies between the round's start (prev) and, of a sample no
 // occluding hit flagged, the round's end (key): where the two decide alike the
-// hit is a fragment or not, and where they differ the warp takes z from the
-// sample's occluding hits of the candidates before it whose b is not above prev
-// (as in the static sampler, where the reason stands).  Flagged samples
-// replay both kinds in order.  640x480, 16 samples, motion blur + depth of
-// field, half of one layer transparent: 16.6 ms on the ordered kernel (one
-// sample per lane, slices one after another, one CTA per SM), 4.7 ms here.
+// hit is a fragment or not.  Where they differ it is none if the sample's
+// nearest occluder comes before it (ids ascend in insertion order); else its
+// lane takes z from the occluding hits of the candidates before it whose b is
+// not above prev (as in the static sampler, where the reason stands).  With a
+// warp per such hit, and without the look at the nearest occluder, frames
+// whose transparent surfaces mostly lie behind opaque ones of the same round
+// were slower than on the ordered kernel (259x138, 36 samples, motion blur +
+// depth of field, one grid in five transparent: 2.38 ms there, 3.28 with a
+// warp per hit, 2.05 now).  Flagged samples replay both kinds in order.
+// 640x480, 16 samples, motion blur + depth of field, half of one layer
+// transparent: 16.6 ms on the ordered kernel (one sample per lane, slices one
+// after another, one CTA per SM), 4.7 ms here.
 __device__ __forceinline__ unsigned long long depth_key_m(float z, int w) {
 	const uint32_t u = __float_as_uint(z);
 	const uint32_t o = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -1260,6 +1266,24 @@ __device__ __forceinline__ int mb_hits(const FrameParams& fp, const GridsDev& g,
 		++n;
 	}
 	return n;
+}
+
+// Do the record's key bounds all lie to one side of the sample, give or take
+// the rounding of bounds between keys (the bound test of mb_sample then fails at
+// any time)?  NaN is on no side.
+template <class R>
+__device__ __forceinline__ bool mb_outside(const R& r, float2 pos, float2 lens) {
+	const float cx = fmaxf(fabsf(r.cocmin[0]), fabsf(r.cocmax[0])) * fabsf(lens.x);
+	const float cy = fmaxf(fabsf(r.cocmin[1]), fabsf(r.cocmax[1])) * fabsf(lens.y);
+	const float mx = cx + 0.01f + 1e-5f * (fabsf(pos.x) + cx), my = cy + 0.01f + 1e-5f * (fabsf(pos.y) + cy);
+	bool left = true, right = true, above = true, below = true;
+	for (int k = 0; k < r.nkeys; ++k) {
+		left = left && r.kbmn[k][0] > pos.x + mx;
+		right = right && r.kbmx[k][0] < pos.x - mx;
+		above = above && r.kbmn[k][1] > pos.y + my;
+		below = below && r.kbmx[k][1] < pos.y - my;
+	}
+	return left || right || above || below;
 }
 
 template <class R>
@@ -1612,10 +1636,11 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 						if (TRANSP && ph == 1) {
 							// kept when !(b > z) and !(z <= D) for the z of the ordered
 							// sequence, which lies between the round's start and its end
-							const float zp = key_depth_m(sm.prev[s]), zk = key_depth_m(sm.key[s]);
+							const unsigned long long kk = sm.key[s];
+							const float zp = key_depth_m(sm.prev[s]), zk = key_depth_m(kk);
 							if (!(zp <= D)) {
 								app = !(wz[lane] > zk) && !(zk <= D);
-								amb = !app;
+								amb = !app && key_winner_m(kk) > r.id;
 							}
 						} else if (NEAR) {
 							const float b = wz[lane];
@@ -1640,32 +1665,39 @@ sample_mbq_kernel(const __grid_constant__ FrameParams fp, const __grid_constant_
 					}
 				}
 				if (TRANSP && ph == 1) {
-					// between the two: z from the occluding candidates before this one
-					uint32_t am = __ballot_sync(0xffffffffu, amb);
-					while (am) {
-						const int src = __ffs(am) - 1;
-						am &= am - 1u;
-						const int s_ = __shfl_sync(0xffffffffu, s, src), c_ = __shfl_sync(0xffffffffu, c, src);
-						const int pl = s_ / spp, j = s_ - pl * spp;
+					// between the two: z from the occluding candidates before this
+					// one, a lane per hit.  Those whose keys' bounds all lie to one
+					// side of the sample are left out first, so that the lanes test
+					// the few others together.
+					if (__ballot_sync(0xffffffffu, amb)) {
+						static_assert(!TRANSP || SLOTS <= 64, "a bit per candidate");
+						const int pl = s / spp, j = s - pl * spp;
 						const int px = tpx0 + pl % fp.tile_w, py = tpy0 + pl / fp.tile_w;
-						const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
-						const float2 d = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s_]);
-						const float zp = key_depth_m(sm.prev[s_]);
+						unsigned long long near_c = 0;
+						float2 xy = make_float2(0.0f, 0.0f), lens = xy;
+						float zp = 0.0f;
+						if (amb) {
+							const float2 o = __ldg(smp.pos + (long long)sm.patidx[pl] * spp + j);
+							xy = make_float2((float)px + o.x, (float)py + o.y);
+							lens = lens_offset(smp, sm.dofidx[pl], spp, sm.kinv[s]);
+							zp = key_depth_m(sm.prev[s]);
+							for (int cc = 0; cc < c; ++cc)
+								if ((sm.rec[cc].bits & 2) && !mb_outside(sm.rec[cc], xy, lens)) near_c |= 1ull << cc;
+						}
 						float z = zp;
-						for (int c0 = 0; c0 < c_; c0 += 32) {
-							const int cc = c0 + lane;
+						while (__ballot_sync(0xffffffffu, near_c != 0)) {
+							if (near_c == 0) continue;
+							const int cc = __ffsll((long long)near_c) - 1;
+							near_c &= near_c - 1;
 							float Dc, bz;
 							float2 uvc;
-							if (cc < c_ && (sm.rec[cc].bits & 2) &&
-							    mb_hits_call(fp, g, smp, bb, sm.rec[cc], slice_times, sm.dofb[sm.kinv[s_]], px, py, j,
-							            make_float2((float)px + o.x, (float)py + o.y), sm.stime[s_], d, INFINITY, Dc, uvc,
-							            bz) > 0 &&
+							if (mb_hits_call(fp, g, smp, bb, sm.rec[cc], slice_times, sm.dofb[sm.kinv[s]], px, py, j, xy, sm.stime[s],
+							                 lens, INFINITY, Dc, uvc, bz) > 0 &&
 							    !(bz > zp))
 								z = fminf(z, Dc);
+							if (z <= D) near_c = 0;  // dropped
 						}
-#pragma unroll
-						for (int k = 16; k > 0; k >>= 1) z = fminf(z, __shfl_xor_sync(0xffffffffu, z, k));
-						if (lane == src) app = !(wz[lane] > z) && !(z <= D);
+						if (amb) app = !(wz[lane] > z) && !(z <= D);
 					}
 					append(app, s, D, sm.rec[c].id, u, v);
 				}
