@@ -314,10 +314,13 @@ filter_kernel(FrameParams fp, SamplerDev smp, SampleStore st, const float* __res
 // half the sums (2 SH + 1 rows of them are live) and twice as many warps fit:
 // the pass waits on loads, not on bandwidth.  Samples are loaded whether or
 // not a window holds them, so a group's records and window words make one
-// round trip.  1920x1080, 64 samples, 3x3: 3.82 ms with a thread per column,
-// 2.22 ms here (14 GB of L2 misses at 6.3 TB/s); 16 samples 658 us on the tile
-// kernel, 399 us here; 935x533, 15 samples, 5x5 with exposure 977 us on the
-// tile kernel, 425 + 23 us here.
+// round trip.  Where windows are tested at sample positions the two lanes test
+// half of a group each (1400x1000, 49 samples, 2x2 filter: 2.42 ms with every
+// test in both lanes, 1.89 here, 2.08 with a thread per column).  1920x1080,
+// 64 samples, 3x3: 3.82 ms with a thread per column, 2.22 ms here (14 GB of L2
+// misses at 6.3 TB/s); 16 samples 658 us on the tile kernel, 399 us here;
+// 935x533, 15 samples, 5x5 with exposure 977 us on the tile kernel, 425 + 23
+// us here.
 struct FiltSum {
 	float acc[4];
 	float gTot;
@@ -334,15 +337,17 @@ constexpr int kRollThreads = 128;  // threads per CTA: half as many display colu
 constexpr int kRollCols = kRollThreads / 2;
 
 // Display rows per CTA: a longer run reads fewer rows twice, a shorter one
-// makes more CTAs; the most rows that leave `per_sm` CTAs for every SM.
+// makes more CTAs; the most rows that leave at least `least` of them.
 // Measured (us, rows 1 / 2 / 4 / 8 / 16): 1920x1080, 16 samples, 3x3: 884 / 605
 // / 486 / 436 / 399; 640x480: 137 / 96 / 77 / 94 / 157; 320x240, 4 samples: 15 /
 // 15 / 20 / 32 / 56; 935x533, 15 samples, 5x5: 1152 / 702 / 507 / 425 / 499 and
 // its three output variables 753 / 441 / 413 / 306 / 439 (half as many CTAs for
-// the same rows: three per SM, the colours four).
-inline int roll_rows(int cols, int h, int nsm, int per_sm) {
+// the same rows: three per SM, the colours four).  5x5 windows read more rows
+// twice, so that a CTA in 32 fewer is worth eight rows to them (640x480, 16
+// samples: 307 us with four, 247 with the 600 CTAs of eight).
+inline int roll_rows(int cols, int h, int least) {
 	int rows = 16;
-	while (rows > 1 && (long long)cols * ((h + rows - 1) / rows) < (long long)per_sm * nsm) rows >>= 1;
+	while (rows > 1 && (long long)cols * ((h + rows - 1) / rows) < least) rows >>= 1;
 	return rows;
 }
 
@@ -452,7 +457,23 @@ __device__ __forceinline__ void roll_steps(const FrameParams& fp, const SamplerD
 						valid[j] = (w & kMaskValid) != 0u;
 						in[j] = ok ? w : 0u;
 					} else {
-						in[j] = !ok ? 0u : (allin ? (1u << W) - 1u : roll_inside<SH>(fp, __ldg(pos + i), (float)px, fpy, xcent, r));
+						in[j] = ok ? (1u << W) - 1u : 0u;
+					}
+				}
+				if (!MASK && !allin) {
+					// the two lanes of a column test two of the four positions each
+					uint32_t mine[2], theirs[2];
+#pragma unroll
+					for (int j = 0; j < 2; ++j) {
+						const int i = i0 + (opac ? 2 : 0) + j;
+						const bool ok = (SPP > 0 && SPP % 4 == 0) || i < spp;
+						mine[j] = ok ? roll_inside<SH>(fp, __ldg(pos + i), (float)px, fpy, xcent, r) : 0u;
+						theirs[j] = __shfl_xor_sync(0xffffffffu, mine[j], 1);
+					}
+#pragma unroll
+					for (int j = 0; j < 2; ++j) {
+						in[j] = opac ? theirs[j] : mine[j];
+						in[2 + j] = opac ? mine[j] : theirs[j];
 					}
 				}
 #pragma unroll
@@ -841,16 +862,18 @@ static void launch_filter_sums(const FrameParams& fp, const SamplerDev& sm, cons
 	// filter is latency-bound: fewer tiles in flight, whose samples would stay
 	// in L2 between the passes, measured slower)
 	const int taps = (2 * fp.shiftX + 1) * (2 * fp.shiftY + 1) * fp.spp;
-	const int cols = (w + kRollCols - 1) / kRollCols, rows = roll_rows(cols, h, nsm, 4);
+	const int cols = (w + kRollCols - 1) / kRollCols, rows = roll_rows(cols, h, (fp.shiftX == 2 ? 31 : 32) * nsm / 8);
 	if (fp.shiftX == fp.shiftY && (fp.shiftX == 1 || fp.shiftX == 2) && taps <= kRollTaps &&
-	    !(rows < 4 && fp.spp <= 16)) {
+	    !(rows < 4 && fp.spp <= 16) && !(fp.shiftX == 2 && fp.spp == 4)) {
 		// 3x3 windows: the rolling window reads each sample three times, not
 		// nine, 5x5 five instead of 25.  Runs of fewer than four rows (images
 		// below about 400x400) lose that where pixels hold few samples
 		// (320x240, 4 samples, 3x3: 12 us on the tile kernel, 15 here; 15
 		// samples, 5x5: 127 and 178), and the tile kernel takes them; with more
 		// samples they gain here too (480x300, 36 samples, 3x3: 332 us against
-		// 129; 211x171, 42 samples, 5x5: 277 against 262)
+		// 129; 211x171, 42 samples, 5x5: 277 against 262).  5x5 windows of 4
+		// samples stay there at any size, where the sample count is a constant
+		// (1400x1000: 270 us there, 436 here; other counts gain here)
 		const dim3 rg(cols, (h + rows - 1) / rows);
 		auto go = [&](auto kernel) { kernel<<<rg, kRollThreads, 0, s>>>(fp, sm, st, ftab, channels, q8, rows); };
 		if (fp.shiftX == 1) {
@@ -905,7 +928,7 @@ void launch_filter_aov(const FrameParams& fp, const SamplerDev& sm, const Sample
 		aov_vertex_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, st.aovsrc, npix, fp.spp);
 		const int sh = fp.shiftX;
 		if (sh == fp.shiftY && (sh == 1 || sh == 2) && (2 * sh + 1) * (2 * sh + 1) * fp.spp <= kRollTaps) {
-			const int cols = (w + kRollThreads - 1) / kRollThreads, rows = roll_rows(cols, h, nsm, 3);
+			const int cols = (w + kRollThreads - 1) / kRollThreads, rows = roll_rows(cols, h, 3 * nsm);
 			const dim3 rg(cols, (h + rows - 1) / rows);
 			for (int k0 = 0; k0 < g.naov; k0 += 4) {
 				const int na = std::min(4, g.naov - k0);
