@@ -634,8 +634,8 @@ aqh_status aqh_set_samples(aqh_ctx* ctx, const aqh_samples* s) {
 		// (a negative entry is a large unsigned one)
 		if (largest(reinterpret_cast<const uint32_t*>(s->shuffle), np) >= (uint32_t)fp.spp)
 			for (size_t i = 0; i < np; ++i)
-			if (s->shuffle[i] < 0 || s->shuffle[i] >= fp.spp)
-				return ctx->fail(AQH_EINVAL, "lens shuffle entry %d out of range", s->shuffle[i]);
+				if (s->shuffle[i] < 0 || s->shuffle[i] >= fp.spp)
+					return ctx->fail(AQH_EINVAL, "lens shuffle entry %d out of range", s->shuffle[i]);
 	}
 	SamplerDev& m = ctx->smp;
 	std::memset(&m, 0, sizeof m);
@@ -1990,7 +1990,7 @@ aqh_status aqh_autotune(aqh_ctx* ctx, int repeats, aqh_tuning* best) {
 				}
 			}
 	// the filter's tiles in flight, with the sampling shape chosen above
-	// (device time of the filter and quantize stage)
+	// (device time of the filter and quantize stage), where it heeds them
 	auto filter_ms = [&](int fc, float& out) -> aqh_status {
 		ctx->tune = pick;
 		ctx->tune.filter_ctas_per_sm = fc;
@@ -2006,7 +2006,9 @@ aqh_status aqh_autotune(aqh_ctx* ctx, int repeats, aqh_tuning* best) {
 	aqh_status fst = filter_ms(0, fbest);
 	int fpick = 0;
 	for (int fc : {3, 4, 5}) {
-		if (fst != AQH_OK) break;
+		FrameParams asked = ctx->fp;
+		asked.filter_ctas = fc;
+		if (fst != AQH_OK || !filter_tiles_asked(asked)) break;
 		float m = 0.0f;
 		fst = filter_ms(fc, m);
 		if (fst == AQH_OK && m < fbest * 0.99f) {

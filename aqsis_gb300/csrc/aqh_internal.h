@@ -305,6 +305,10 @@ aqh_status resolve_frame(const aqh_frame_desc& d, FrameParams& fp, std::vector<f
 void set_tiling(FrameParams& fp, int tile_pixels = 0, int supertile_px = 0);
 void dof_bounds_h(int xs, int ys, std::vector<float4>& out);
 constexpr int kRollTaps = 9 * AQH_MAX_SPP_DEV;  // filter weights the rolling filters hold at most
+// Does the frame's filter heed aqh_tuning::filter_ctas_per_sm?
+inline bool filter_tiles_asked(const FrameParams& fp) {
+	return fp.filter_ctas > 0 && !(fp.shiftX == 1 && fp.shiftY == 1 && fp.spp > 16);
+}
 // Does the frame keep a window word per sample (SampleStore::wmask)?
 bool window_words(const FrameParams& fp);
 // `q8` (may be null): the frame's r g b a display quantized to 8 bits,

@@ -864,7 +864,7 @@ static void launch_filter_sums(const FrameParams& fp, const SamplerDev& sm, cons
 	const int taps = (2 * fp.shiftX + 1) * (2 * fp.shiftY + 1) * fp.spp;
 	const int cols = (w + kRollCols - 1) / kRollCols, rows = roll_rows(cols, h, (fp.shiftX == 2 ? 31 : 32) * nsm / 8);
 	if (fp.shiftX == fp.shiftY && (fp.shiftX == 1 || fp.shiftX == 2) && taps <= kRollTaps &&
-	    !(rows < 4 && fp.spp <= 16) && !(fp.shiftX == 2 && fp.spp == 4)) {
+	    !(rows < 4 && fp.spp <= 16) && !(fp.shiftX == 2 && fp.spp == 4) && !filter_tiles_asked(fp)) {
 		// 3x3 windows: the rolling window reads each sample three times, not
 		// nine, 5x5 five instead of 25.  Runs of fewer than four rows (images
 		// below about 400x400) lose that where pixels hold few samples

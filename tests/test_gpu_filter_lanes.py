@@ -28,3 +28,17 @@ def test_position_tests_match_oracle(hider, oracle, filt, fw, xs, ys, outside):
 def test_kernel_choice_matches_oracle(hider, oracle, w, h, xs, ys, fw):
     sc = _scene(w, h, xs, ys, "mitchell", fw, 0, seed=w + h)
     compare(hider.render_scene(sc), oracle.render(sc), exact_pixels=True)
+
+
+@pytest.mark.parametrize("xs,ys,fw", [(4, 4, 2.0), (4, 4, 3.0), (5, 3, 4.0), (6, 6, 5.0), (6, 6, 2.0)])
+def test_asking_for_tiles_changes_no_pixel(aqh_lib, oracle, xs, ys, fw):
+    """filter_ctas_per_sm makes windows that would roll go by tiles."""
+    sc = _scene(300, 411, xs, ys, "catmull-rom", fw, 0, seed=xs)
+    ref = oracle.render(sc)
+    h = aqh_lib.Hider(0)
+    try:
+        for ctas in (0, 1, 8):
+            h.set_tuning(filter_ctas_per_sm=ctas)
+            compare(h.render_scene(sc), ref, exact_pixels=True)
+    finally:
+        h.close()
