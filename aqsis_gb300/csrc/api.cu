@@ -439,7 +439,6 @@ struct aqh_ctx {
 	SamplerDev smp{};
 	bool samples_set = false;
 	int64_t frag_capacity = 0;
-	bool debug_samples = true;
 	aqh_frame_stats stats{};
 	int64_t st_list_cap = 0;
 
@@ -1219,14 +1218,14 @@ static aqh_status plan_render(aqh_ctx* ctx, RenderPlan& P) {
 	store.a = ctx->d_sa.as<float4>();
 	store.b = ctx->d_sb.as<float4>();
 	if (wmask) store.wmask = ctx->d_wmask.as<uint32_t>();
-	if (ctx->debug_samples) {
-		AQH_TRY(ctx->d_win.ensure(P.nsamp * 4), "alloc");
-		AQH_TRY(ctx->d_oz.ensure(P.nsamp * 4), "alloc");
-		AQH_TRY(ctx->d_nf.ensure(P.nsamp * 4), "alloc");
-		store.winner = ctx->d_win.as<int32_t>();
-		store.occlz = ctx->d_oz.as<float>();
-		store.nfrag = ctx->d_nf.as<int32_t>();
-	}
+	// aqh_read_samples returns these; the mixed sampler hands its occluding
+	// hits to Combine in the first two
+	AQH_TRY(ctx->d_win.ensure(P.nsamp * 4), "alloc");
+	AQH_TRY(ctx->d_oz.ensure(P.nsamp * 4), "alloc");
+	AQH_TRY(ctx->d_nf.ensure(P.nsamp * 4), "alloc");
+	store.winner = ctx->d_win.as<int32_t>();
+	store.occlz = ctx->d_oz.as<float>();
+	store.nfrag = ctx->d_nf.as<int32_t>();
 	if (fp.midpoint_store) {
 		AQH_TRY(ctx->d_hz.ensure(P.nsamp * 4), "alloc");
 		store.hitz = ctx->d_hz.as<float>();
@@ -2173,7 +2172,6 @@ aqh_status aqh_read_samples(aqh_ctx* ctx, int32_t* winner, float* occlz, int32_t
 	const FrameParams& fp = ctx->fp;
 	const size_t n = (size_t)fp.sw * fp.sh * fp.spp;
 	if (nsamples < n) return ctx->fail(AQH_EINVAL, "buffers hold %zu samples, %zu needed", nsamples, n);
-	if (!ctx->debug_samples && (winner || occlz || nfrag)) return ctx->fail(AQH_EINVAL, "debug sample outputs are off");
 	cudaSetDevice(ctx->device);
 	cudaStream_t s = ctx->stream;
 	if (winner) AQH_TRY(cudaMemcpyAsync(winner, ctx->d_win.p, n * 4, cudaMemcpyDeviceToHost, s), "read");

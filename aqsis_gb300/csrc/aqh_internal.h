@@ -150,14 +150,14 @@ __host__ __device__ inline size_t store_size(long long npix, int spp) {
 
 constexpr uint32_t kMaskValid = 0x80000000u;  // SampleStore::wmask: the sample holds a hit
 
-// a and b in the store layout above; the debug arrays are pixel-major
+// a and b in the store layout above; winner, occlz and nfrag are pixel-major
 // ([pixel][sample index]).
 struct SampleStore {
 	float4* a;        // r, g, b, depth
 	float4* b;        // or, og, ob, valid (1.0f / 0.0f)
-	int32_t* winner;  // debug: occluding hit id before Combine (or null)
-	float* occlz;     // debug: occlZ (or null)
-	int32_t* nfrag;   // debug: transparent fragment count (or null)
+	int32_t* winner;  // occluding hit id before Combine (null in the no-allocation form)
+	float* occlz;     // occlZ (or null)
+	int32_t* nfrag;   // transparent fragment count (or null)
 	float* hitz;      // depth of the occluding hit when occlZ tracks the second-nearest
 	                  // depth (midpoint depth filter with a z display), else null
 	uint32_t* wmask;  // per sample (store layout): bit (fy + shiftY) * (2 shiftX + 1) + fx + shiftX set

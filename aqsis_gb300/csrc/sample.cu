@@ -1804,7 +1804,7 @@ void launch_sample_tiles_q(const FrameParams& fp, const GridsDev& g, const Sampl
 	if (colours_ready && !split) cudaStreamWaitEvent(s, colours_ready, wait_flags);
 	// transparent frames with one occlZ per sample and no solids: the mixed
 	// sampler takes them when they have occluders, else the ordered kernel does
-	const bool mixed = transp && fp.frag_only && fp.cullable && g.csg.nnodes == 0 && pool.heads && st.winner && st.occlz;
+	const bool mixed = transp && fp.frag_only && fp.cullable && g.csg.nnodes == 0 && pool.heads;
 	if (transp && fp.frag_only) {
 		// both samplers are queued; each reads the occluder flag and one returns at once
 		if (fp.cullable) {
