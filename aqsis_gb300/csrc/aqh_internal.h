@@ -215,7 +215,11 @@ struct BinBuffers {
 constexpr int kIrrWords = 32;     // grids of more micropolygons than bits are not analysed
 constexpr int kRedoHead = 5;      // counters in front of the redo entries
 constexpr int kRedoPerTile = 8;   // redo entries of a tile at most (more pixels: the whole tile)
-constexpr int64_t kListBound = 1 << 21;  // list entries (8 MB) a plain frame reserves without asking for their number
+// List entries (8 MB, twice in opaque frames) a plain frame reserves without
+// asking for their number.  Not waiting for it saves 15 to 20 us of a call at any
+// size: 304 -> 287 us at 320x240, 2011 -> 1994 at 2.0M entries, but 0.5% of it
+// where the bound would be 35 MB (1920x1080, 60,000 grids 3863 -> 3845).
+constexpr int64_t kListBound = 1 << 21;
 // List entries a batched frame reserves at first: 16 super-tiles per grid.
 inline int64_t list_batched(int64_t ngrids) { return ngrids * 16 + 4096; }
 // The most entries either form reserves before it knows their number.

@@ -451,24 +451,24 @@ void launch_st_count(const FrameParams& fp, const GridsDev& g, BinBuffers& b, cu
 //
 // The depth of a hit is the bilinear mix of the corner depths at the (u, v) of
 // two Newton steps from the centre C.  With M1 = E + G/2, M2 = F + G/2, area A
-// = M1 x M2 and G = g1 M1 + g2 M2, the first step lands at (x, y) = (u - 1/2, v
-// - 1/2) with M1 x + M2 y = P - C, affine in the sample position P: at the
+// = M1 x M2 and G = g1 M1 + g2 M2, the first step lands at (x, y) = (u - 1/2,
+// v - 1/2) with M1 x + M2 y = P - C, affine in the sample position P: at the
 // corners x = +-1/2 +- g1/4 and y = +-1/2 +- g2/4, so |x| <= X = 1/2 + |g1|/4
 // and |y| <= Y over the corners' hull, which holds every point the edge tests
 // accept.  The second step's determinant there is A (1 + g2 x + g1 y), also
 // affine, so at least A kappa with kappa its least value at the corners, 1 +-
 // (g1 + g2)/2 + g1 g2/2 and 1 +- (g1 - g2)/2 - g1 g2/2, and its step is -(g1,
-// g2) x y / (det / A).  Hence |u - 1/2| <= U = X + |g1| X Y /
-// kappa, V alike, the weights' absolute values sum to at most W = max(1, 2U)
-// max(1, 2V), the negative ones to (W - 1)/2, and the depth is at least min z -
-// (W - 1)/2 (max z - min z).  Rounding: positions carry 2^-20 of the
-// coordinates into the steps (eta below; a step divides it by kappa), the edge
-// tests accept points up to 2^-10 / c < 1/32 of a cell outside for quads with
-// 32 A >= L^2 (L the extent) whose corners turn by at least c A, c = 1 - (|g1| +
-// |g2|)/2 >= 0.05, and the mix itself rounds by 2^-19 W max|z|.  Quads with
-// kappa < 0.05 or c < 0.05 (folded, nearly singular: one in 2,000 of a grid of
-// unit spacing and +-0.3 jitter), thin ones and anything not finite are
-// irregular.
+// g2) x y / (det / A).  Hence |u - 1/2| <= U = X + |g1| X Y / kappa, V alike,
+// the weights' absolute values sum to at most W = max(1, 2U) max(1, 2V), the
+// negative ones to (W - 1)/2, and the depth is at least min z - (W - 1)/2 (max
+// z - min z).  (The bound below charges W/2, half a depth range more than
+// that.)  Rounding: positions carry 2^-20 of the coordinates into the steps
+// (eta below; a step divides it by kappa), the edge tests accept points up to
+// 2^-10 / c < 1/32 of a cell outside for quads with 32 A >= L^2 (L the extent)
+// whose corners turn by at least c A, c = 1 - (|g1| + |g2|)/2 >= 0.05, and the
+// mix itself rounds by 2^-19 W max|z|.  Quads with kappa < 0.05 or c < 0.05
+// (folded, nearly singular: one in 2,000 of a grid of unit spacing and +-0.3
+// jitter), thin ones and anything not finite are irregular.
 //
 // Corners that move (rho > 0) are within rho, per coordinate, of a translate of
 // the given ones: E and F then move by 2 rho, G, M1 and M2 by 4 rho, and the

@@ -553,7 +553,6 @@ __device__ __forceinline__ bool stage_mb(const FrameParams& fp, const GridsDev& 
                                          int tpx0, int tpy0, int tpx1, int tpy1, int lend, int& lp, int& r0,
                                          int& qtotal, int& npend, const float* blk = nullptr) {
 	const int t = threadIdx.x;
-	const bool usingDof = fp.use_dof != 0;
 	while (npend < kSlots) {
 		if (r0 >= qtotal) {
 			if (lp >= lend) return true;
@@ -624,13 +623,12 @@ __device__ __forceinline__ bool stage_mb(const FrameParams& fp, const GridsDev& 
 			}
 			gid = sm.qgrid[lo];
 			m = p - sm.qcum[lo];
-			const int cu = __ldg(g.cu + gid), nk = __ldg(g.nkeys + gid);
+			const int cu = __ldg(g.cu + gid);
 			const int sub = sm.qsub[lo];
 			if (sub >= 0) {
 				const int w = sub >> 16;
 				m = (((sub >> 8) & 0xff) + m / w) * cu + ((sub & 0xff) + m % w);
 			}
-			(void)nk;
 			// conservative pixel rectangle over every time slice and lens stratum
 			const int4* pb = bb.mp_bounds ? bb.mp_bounds + (__ldg(g.mpbase + gid) + m) * bb.mp_stride : nullptr;
 			const MbStageBound sb = pb ? unpack_stage_bound(__ldg(pb)) : mb_stage_bound(fp, g, gid, m);

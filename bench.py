@@ -543,9 +543,8 @@ def run_gpu(args):
     pk = peaks()
     alg_bytes = g.nbytes_algorithmic()  # P + Ci + Oi float4 per vertex, read once
     # DRAM bytes (read + write) of one sampler launch from an ncu capture of the
-    # same kernel on a smaller frame of the same stream, scaled by micropolygons
-    # (profiles/sample_near_kernel_opaque_stream_scale035.md); None where no
-    # capture of that kernel exists
+    # same kernel (sample_near_kernel) on a smaller frame of the same stream,
+    # scaled by micropolygons; None where no capture of that kernel exists
     traffic = TRAFFIC_PER_MP[args.workload] * mps if TRAFFIC_PER_MP.get(args.workload) else None
     ms_sample = r["stage"]["sample"]
     achieved = alg_bytes / (ms_sample / 1e3) / 1e9
