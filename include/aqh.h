@@ -252,7 +252,8 @@ aqh_status aqh_render(aqh_ctx* ctx, int sync);
  * list size where grids times super-tiles exceed 2^21 (smaller frames reserve
  * room for that many list entries); it returns once the frame's host arrays
  * have been read.  BATCHED:
- * a persistent sampling kernel pulls tiles from a device work queue, nothing
+ * a persistent sampling kernel pulls tiles from a device work queue (opaque
+ * frames too small for it launch a block per tile), nothing
  * synchronizes with the host inside a frame, and the frame's whole
  * bin -> sample -> filter -> quantize sequence is one CUDA graph, captured on
  * the first render and replayed while the frame's arguments are unchanged;
