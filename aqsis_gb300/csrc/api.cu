@@ -1109,6 +1109,15 @@ static aqh_status inputs_read(aqh_ctx* ctx) {
 	return AQH_OK;
 }
 
+// A frame that cannot be rendered: the caller may free its arrays, some of
+// which may be on their way.
+static aqh_status abandon_frame(aqh_ctx* ctx, aqh_status st) {
+	const std::string why = ctx->err;
+	if (cudaEventRecord(ctx->ev_inputs, ctx->stream) == cudaSuccess) inputs_read(ctx);
+	ctx->err = why;
+	return st;
+}
+
 // Is the frame large enough for near to far sampling?  The order, the depth
 // bounds and the second sampler are four launches more (three in moving
 // frames), 10 to 15 us that the hidden micropolygons have to be worth.  Static
@@ -1709,25 +1718,21 @@ aqh_status aqh_render(aqh_ctx* ctx, int sync) {
 	// so do frames with trim curves (their micropolygon marks are per frame)
 	const bool batched = ctx->mode == AQH_MODE_BATCHED && P.g.csg.nnodes == 0 && P.g.trim.nsets == 0 && !ctx->cull_on;
 	const bool whole = sync != 0 || (!batched && P.g.csg.nnodes > 0);  // wait for the whole frame
-	if (st != AQH_OK || (!whole && (!batched || ctx->staged_in_use)))
+	if (st == AQH_OK && !whole && (!batched || ctx->staged_in_use))
 		AQH_TRY(cudaEventRecord(ctx->ev_inputs, ctx->stream), "uploads");
-	if (st != AQH_OK) {
-		inputs_read(ctx);
-		return st;
-	}
+	if (st != AQH_OK) return abandon_frame(ctx, st);
 	ctx->stats.micropolygons = P.nmps;
 	ctx->stats.samples = (int64_t)P.nsamp;
 	ctx->stats.grids = P.g.ngrids;
 	st = batched ? render_batched(ctx, P, whole) : render_plain(ctx, P, whole);
+	if (st != AQH_OK) return abandon_frame(ctx, st);
 	if (whole) {
-		if (st == AQH_OK) ctx->staged_in_use = false;
-		return st;
+		ctx->staged_in_use = false;
+		return AQH_OK;
 	}
-	if (batched) return st;
 	// the caller may reuse its arrays once the plain form returns; by now the
 	// whole frame is queued, so the wait leaves the device no gap
-	const aqh_status in = inputs_read(ctx);
-	return st != AQH_OK ? st : in;
+	return batched ? AQH_OK : inputs_read(ctx);
 }
 
 aqh_status aqh_synchronize(aqh_ctx* ctx) {

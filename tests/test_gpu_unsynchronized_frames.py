@@ -173,3 +173,27 @@ def test_stats_do_not_wait_for_the_frame(aqh_lib):
         del keep
     finally:
         h.close()
+
+
+def test_refused_frame_has_read_its_arrays(aqh_lib):
+    """Camera-space grids without a matrix are refused after their upload was
+    queued: aqh_render returns once that is done, with its own message."""
+    a = _scene(5)
+    a.grids.flags = a.grids.flags | np.int32(S.GRID_CAMERA)
+    pin = _Pinned(aqh_lib.load())
+    h = aqh_lib.Hider(0)
+    try:
+        a.grids.P = pin.copy(a.grids.P)
+        sc, keep = _busy(h)
+        h.frame_begin(a.frame)
+        h.submit_grids_host(a.grids)
+        _set_samples(h, a.samples)
+        with pytest.raises(aqh_lib.AqhError, match="camera-to-raster"):
+            h.render(sync=False)
+        t0 = time.perf_counter()
+        h.synchronize()
+        assert time.perf_counter() - t0 < 1e-3   # the busy frame, and so the upload behind it, was done
+        del keep, sc
+    finally:
+        h.close()
+        pin.free()
